@@ -251,7 +251,7 @@ int adjoint_device(qf_ctx *ctx, uint32_t n, const std::vector<BGate> &gates, con
         }
     } guard{ctx, &ckpt};
     PlanOpts po;
-    default_tiling(n, dtype, o->exec.tile_qubits, &po.tile_qubits, &po.low_qubits);
+    sweep_tiling(n, dtype, &o->exec, false, false, po);
     po.search = !(o->exec.flags & QF_EXEC_FLAG_PLAN_FIRST_COME);
     QF_TRY(fill_zero_state(psi));
     for (size_t s = 0; s < n_seg; ++s) {
@@ -276,6 +276,7 @@ int adjoint_device(qf_ctx *ctx, uint32_t n, const std::vector<BGate> &gates, con
     size_t total_slots = 0;
     {
         PlanOpts bo = po;
+        sweep_tiling(n, dtype, &o->exec, true, false, bo);
         bo.backward = true;
         bo.merge_1q = true;
         // the dual passes (psi and lambda per tile) are bound by arithmetic, not
@@ -1005,7 +1006,7 @@ int qf_sv_apply_ops(qf_sv *sv, const qf_op *ops, uint64_t n_ops, const double *p
     std::vector<BGate> gates;
     QF_TRY(bind_ops(sv->n, ops, n_ops, params, n_params, inputs, n_inputs, -1, 0.0, gates));
     QF_TRY(bind_device(sv->ctx));
-    return execute_gates(sv, gates, opts);
+    return execute_gates(sv, gates, opts, n_params == 0 && n_inputs == 0);
 }
 
 int qf_sv_norm_sqr(qf_sv *sv, double *out) {
@@ -2030,9 +2031,10 @@ int qf_adjoint_plan_stats(uint32_t qubits, int dtype, const qf_op *ops, uint64_t
     }
     const size_t n_seg = seg_begin.size();
     PlanOpts po;
-    default_tiling(qubits, dtype, opts->exec.tile_qubits, &po.tile_qubits, &po.low_qubits);
+    sweep_tiling(qubits, dtype, &opts->exec, false, false, po);
     po.search = !(opts->exec.flags & QF_EXEC_FLAG_PLAN_FIRST_COME);
     PlanOpts bo = po;
+    sweep_tiling(qubits, dtype, &opts->exec, true, false, bo);
     bo.backward = true;
     bo.merge_1q = true;
     bo.search = false;
@@ -2079,7 +2081,7 @@ int qf_plan_stats(uint32_t qubits, int dtype, const qf_op *ops, uint64_t n_ops, 
         return QF_OK;
     }
     PlanOpts po;
-    QF_TRY(plan_opts_for(qubits, dtype, opts, po));
+    QF_TRY(plan_opts_for(qubits, dtype, opts, n_params == 0 && n_inputs == 0, po));
     Plan plan;
     QF_TRY(plan_passes(qubits, gates, po, plan));
     *n_passes = plan.passes.size();

@@ -6,10 +6,12 @@
 #include <complex>
 #include <cstring>
 #include <string>
+#include <memory>
 #include <mutex>
-#include <map>
+#include <unordered_map>
 
 #include "qf_internal.h"
+#include "vm.h"
 
 namespace qf {
 
@@ -211,13 +213,36 @@ void default_tiling(uint32_t n, int dtype, int requested_tile, int *tile, int *l
     *low = lo;
 }
 
-// Tiling of forward sweeps. Compiled passes also run on 13-qubit tiles when a
-// caller asks for them (one CTA of 512 threads per SM: 18 % fewer passes on the
-// 30-qubit circuit but 33 % slower passes, latency-bound), so the default stays
-// at 12.
-void forward_tiling(uint32_t n, int dtype, int requested_tile, int flags, int *tile, int *low) {
-    (void)flags;
-    default_tiling(n, dtype, requested_tile, tile, low);
+// Planning options of a sweep under a caller's qf_exec_opts: which engine runs
+// it and the tile that engine wants.
+//  * compiled passes (complex64 from kJitMinQubits qubits, or on request): 12
+//    qubits over the low five. 13 on request (one CTA of 512 threads per SM: 18 %
+//    fewer passes on the 30-qubit circuit but 33 % slower ones, latency-bound).
+//  * register-tile passes (vm.h): complex128, and the gate lists applied to a
+//    resident complex64 state (`resident`) below kJitMinQubits, on 6 to 12 qubits
+//    (a smaller state whole). Wider requests run at the widest.
+//  * complex64 otherwise: calls whose results leave as f64 (parameterised runs,
+//    energies, gradients, density matrices, shots) are promised to reproduce
+//    earlier results to f64 accuracy, which a pass that orders its float32
+//    operations differently cannot: the in-order passes (rspass.cu, sweep.cu) stay.
+//  * the shared-memory interpreter for the rest (dense blocks, on request).
+void sweep_tiling(uint32_t n, int dtype, const qf_exec_opts *opts, bool dual, bool resident, PlanOpts &po) {
+    const int req = opts ? opts->tile_qubits : 0, flags = opts ? opts->flags : 0;
+    default_tiling(n, dtype, req, &po.tile_qubits, &po.low_qubits);
+    po.merge_any = po.vm = false;
+    if ((opts && opts->block_qubits >= 2 && !dual) || (flags & QF_EXEC_FLAG_SMEM_TILES)) return;
+    if (dtype == QF_C64) {
+        if (!resident) return;
+        const bool jit = !(flags & QF_EXEC_FLAG_NO_JIT) && ((flags & QF_EXEC_FLAG_JIT) || n >= kJitMinQubits);
+        if (jit && n >= 12 && jit_available()) return;
+    }
+    const int widest = vm_widest(dtype, dual);
+    int k = req > 0 ? std::min(req, widest) : vm_default_tile(n, dtype, dual);
+    k = std::min(k, (int)n);
+    if (k < 6 && k != (int)n) return;
+    po.tile_qubits = k;
+    po.low_qubits = std::min(k, dtype == QF_C64 ? 4 : 3);  // 128-byte runs
+    po.merge_any = po.vm = true;
 }
 
 namespace {
@@ -564,9 +589,8 @@ struct PassChoice {
 };
 std::string plan_key_of(uint32_t n, int k, int low, const PlanOpts &o, const std::vector<Item> &items) {
     std::string key;
-    auto put = [&](uint64_t v, int bytes) {
-        for (int b = 0; b < bytes; ++b) key.push_back((char)((v >> (8 * b)) & 0xFF));
-    };
+    key.reserve(16 + 11 * items.size());
+    auto put = [&](uint64_t v, int bytes) { key.append(reinterpret_cast<const char *>(&v), (size_t)bytes); };
     put(n, 1);
     put((uint64_t)k, 1);
     put((uint64_t)low, 1);
@@ -582,25 +606,24 @@ std::string plan_key_of(uint32_t n, int k, int low, const PlanOpts &o, const std
     }
     return key;
 }
+using PassChoices = std::shared_ptr<const std::vector<PassChoice>>;
 struct PlanCache {
     std::mutex mu;
-    std::map<std::string, std::vector<PassChoice>> entries;
+    std::unordered_map<std::string, PassChoices> entries;
 };
 PlanCache &plan_cache() {
     static PlanCache c;
     return c;
 }
-bool plan_cache_get(const std::string &key, std::vector<PassChoice> &out) {
+PassChoices plan_cache_get(const std::string &key) {
     std::lock_guard<std::mutex> lk(plan_cache().mu);
     auto it = plan_cache().entries.find(key);
-    if (it == plan_cache().entries.end()) return false;
-    out = it->second;
-    return true;
+    return it == plan_cache().entries.end() ? nullptr : it->second;
 }
 void plan_cache_put(const std::string &key, std::vector<PassChoice> &&v) {
     std::lock_guard<std::mutex> lk(plan_cache().mu);
     if (plan_cache().entries.size() >= 64) plan_cache().entries.clear();  // bound the host memory
-    plan_cache().entries[key] = std::move(v);
+    plan_cache().entries[key] = std::make_shared<const std::vector<PassChoice>>(std::move(v));
 }
 }  // namespace
 
@@ -618,6 +641,7 @@ int plan_passes(uint32_t n, const std::vector<BGate> &gates, const PlanOpts &o, 
     const int kb = (!o.backward && o.block_qubits >= 2) ? std::min(o.block_qubits, kMaxBlockQubits) : 0;
     if (kb && kb > k) return fail(QF_ERR_INVALID_ARGUMENT, "blocks of %d qubits do not fit a %d-qubit tile", kb, k);
     plan.block_qubits = (uint32_t)kb;
+    plan.vm = o.vm;
     std::vector<Item> items;
     items.reserve(gates.size() * (o.backward ? 2 : 1));
     if (!o.backward) {
@@ -640,12 +664,12 @@ int plan_passes(uint32_t n, const std::vector<BGate> &gates, const PlanOpts &o, 
     // and overlaps (new angles, shifted parameters, another optimiser step)
     // replays the recorded choices instead of searching again.
     const std::string key = plan_key_of(n, k, low, o, items);
-    std::vector<PassChoice> replay;
-    const bool hit = plan_cache_get(key, replay);
+    const PassChoices known = plan_cache_get(key);
+    const bool hit = known != nullptr;
     std::vector<PassChoice> record;
     size_t pass_i = 0;
 
-    while (hit ? pass_i < replay.size() : !remaining.empty()) {
+    while (hit ? pass_i < known->size() : !remaining.empty()) {
         uint64_t L;
         std::vector<Item> taken;
         std::vector<int> last_on(n, -1);  // index into taken of the last item touching q
@@ -663,7 +687,7 @@ int plan_passes(uint32_t n, const std::vector<BGate> &gates, const PlanOpts &o, 
                     // FMAs per amplitude pair, the two apart a real rotation and a
                     // diagonal phase (deferred when its qubit is off the registers).
                     const bool varying = taken[prev].g.varying || it.g.varying;
-                    if (!varying || matrix_is_diag(c) || matrix_is_cheap(c)) {
+                    if (!varying || o.merge_any || matrix_is_diag(c) || matrix_is_cheap(c)) {
                         std::memcpy(taken[prev].g.m, c, sizeof c);
                         taken[prev].g.varying = varying;
                         taken[prev].g.diag = matrix_is_diag(c);
@@ -674,12 +698,12 @@ int plan_passes(uint32_t n, const std::vector<BGate> &gates, const PlanOpts &o, 
             }
             taken.push_back(it);
             const int ti = (int)taken.size() - 1;
-            for (uint32_t q = 0; q < n; ++q)
-                if ((it.touch >> q) & 1ULL) last_on[q] = ti;
+            for (uint64_t m = it.touch; m; m &= m - 1) last_on[__builtin_ctzll(m)] = ti;
         };
         if (hit) {
-            L = replay[pass_i].L;
-            for (int idx : replay[pass_i].sel) take(items[idx]);
+            L = (*known)[pass_i].L;
+            taken.reserve((*known)[pass_i].sel.size());
+            for (int idx : (*known)[pass_i].sel) take(items[idx]);
             ++pass_i;
         } else {
             // The first remaining item must fit: shrink the always-resident low
@@ -794,6 +818,7 @@ int plan_passes(uint32_t n, const std::vector<BGate> &gates, const PlanOpts &o, 
             pscale = 1.0;
             any_factored = false;
         };
+        p.gates.reserve(taken.size());
         for (const Item &it : taken) {
             TileOp t;
             std::memset(&t, 0, sizeof t);
@@ -808,7 +833,7 @@ int plan_passes(uint32_t n, const std::vector<BGate> &gates, const PlanOpts &o, 
                 else if (g.axis == QF_PAULI_Y) { t.kind = T_OVL_Y; t.b0 = (uint8_t)lb0; }
                 else if (lb0 >= 0) { t.kind = T_OVL_ZL; t.b0 = (uint8_t)lb0; }
                 else { t.kind = T_OVL_ZG; t.g0 = g.q0; }
-                plan.ops.push_back(t);
+                if (!o.vm) plan.ops.push_back(t);
                 BGate ov = g;
                 ov.kind = BK_OVL;
                 ov.op_index = t.slot;
@@ -816,6 +841,7 @@ int plan_passes(uint32_t n, const std::vector<BGate> &gates, const PlanOpts &o, 
                 continue;
             }
             p.gates.push_back(g);
+            if (o.vm) continue;  // register-tile passes are lowered from the gates (vmplan.cpp)
             switch (g.kind) {
             case BK_BLOCK: {
                 t.kind = T_BLOCK;
@@ -865,7 +891,7 @@ int plan_passes(uint32_t n, const std::vector<BGate> &gates, const PlanOpts &o, 
         p.a.n_ops = (uint32_t)plan.ops.size() - p.op_begin;
         p.a.n_mats = (uint32_t)(plan.mats.size() / 8) - p.mat_begin;
         p.a.n_slots = plan.n_slots - p.a.slot_base;
-        plan.passes.push_back(p);
+        plan.passes.push_back(std::move(p));
     }
     if (!hit) plan_cache_put(key, std::move(record));
     return QF_OK;

@@ -267,12 +267,15 @@ struct Plan {
     uint32_t n_slots = 0;
     std::vector<double> bmats;       // dense block matrices (interleaved complex), see BK_BLOCK
     uint32_t block_qubits = 0;       // fusion width the plan was made with (0: gates one by one)
+    bool vm = false;                 // for register-tile passes: gates only, no tile ops
 };
 
 struct PlanOpts {
     int tile_qubits = 12;   // k
     int low_qubits = 5;     // always-local contiguous low qubits
     bool merge_1q = true;   // multiply consecutive 1q gates on one qubit
+    bool vm = false;        // the plan is for register-tile passes (vm.h)
+    bool merge_any = false; // even when the product is a general complex matrix (register-tile passes)
     bool backward = false;  // adjoint reverse sweep: inverse gates + overlaps
     int max_items = 768;    // bound on ops per pass (shared-memory budget)
     bool search = true;     // choose each pass's resident qubits by look-ahead
@@ -294,14 +297,15 @@ std::vector<uint32_t> qubits_of_mask(uint64_t m);
 int lower_rs(const Plan &plan, int wb, RsPlan &out);
 // Default tile/low widths for a state.
 void default_tiling(uint32_t n, int dtype, int requested_tile, int *tile, int *low);
-void forward_tiling(uint32_t n, int dtype, int requested_tile, int flags, int *tile, int *low);
+// Tile and engine of a forward (dual: backward) sweep under a caller's options;
+// resident: the gates of qf_sv_apply_ops on a state the caller holds.
+void sweep_tiling(uint32_t n, int dtype, const qf_exec_opts *opts, bool dual, bool resident, PlanOpts &po);
 
 // ---- launchers (kernels in *.cu) ------------------------------------------
 // Unfused single-gate sweeps.
 int launch_gate1(qf_sv *sv, const BGate &g);
 int launch_gate2(qf_sv *sv, const BGate &g);
-// Upload a plan's ops+matrices into the context workspace and run every pass
-// (register-tiled for complex64 where the tile fits, shared memory otherwise).
+// Run every pass of a plan on the engine it was made for (sweep_tiling).
 int run_plan(qf_sv *sv, const Plan &plan, int flags = 0);
 int run_plan_smem(qf_sv *sv, const Plan &plan);
 // Plans with dense blocks: the shared-memory block interpreter (any width,
@@ -310,11 +314,11 @@ int run_plan_smem(qf_sv *sv, const Plan &plan);
 int run_plan_blocks(qf_sv *sv, const Plan &plan);
 bool mma_blocks_fit(const Plan &plan);
 int run_plan_blocks_mma(qf_sv *sv, const Plan &plan);
-int run_plan_rs(qf_sv *sv, const Plan &plan, int wb);
 // Compiled register-tiled passes (jit.cpp); states of at least kJitMinQubits
 // qubits use them by default.
 constexpr uint32_t kJitMinQubits = 24;
 bool jit_available();
+int run_plan_rs(qf_sv *sv, const Plan &plan, int wb);
 int run_plan_jit(qf_sv *sv, const Plan &plan, int wb);
 // Generate the plan's pass kernels and compile them with NVRTC without
 // loading them (no GPU needed); for tests of the code generator. `dual`
@@ -435,8 +439,8 @@ void rng_jump_matrices(uint64_t stride, uint64_t (*mats)[64], int count);
 uint64_t rng_apply(const uint64_t cols[64], uint64_t state);
 
 // Dispatcher for a bound gate list on a resident state.
-int execute_gates(qf_sv *sv, const std::vector<BGate> &gates, const qf_exec_opts *opts);
+int execute_gates(qf_sv *sv, const std::vector<BGate> &gates, const qf_exec_opts *opts, bool resident = false);
 // Planning options of a forward sweep (tile widths, look-ahead, block width).
-int plan_opts_for(uint32_t n, int dtype, const qf_exec_opts *opts, PlanOpts &po);
+int plan_opts_for(uint32_t n, int dtype, const qf_exec_opts *opts, bool resident, PlanOpts &po);
 
 }  // namespace qf

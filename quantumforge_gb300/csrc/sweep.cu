@@ -19,6 +19,7 @@
 
 #include "qf_device.cuh"
 #include "qf_internal.h"
+#include "vm.h"
 
 namespace qf {
 
@@ -795,8 +796,6 @@ int run_plan_smem(qf_sv *sv, const Plan &plan) {
     return launch_passes<double2, false>(sv, nullptr, plan, nullptr);
 }
 
-// complex64 plans with 12- or 13-qubit tiles run register-tiled; the rest
-// (complex128, small states, QF_EXEC_FLAG_SMEM_TILES) in shared memory.
 int run_plan(qf_sv *sv, const Plan &plan, int flags) {
     if (plan.passes.empty()) return QF_OK;
     if (plan.block_qubits) {  // dense k-qubit blocks
@@ -809,10 +808,11 @@ int run_plan(qf_sv *sv, const Plan &plan, int flags) {
         }
         return run_plan_blocks(sv, plan);
     }
+    if (plan.vm) return run_plan_vm(sv, plan);
     if (sv->dtype == QF_C64 && !(flags & QF_EXEC_FLAG_SMEM_TILES) && sv->n >= 12) {
         const uint32_t k = plan.passes[0].a.k;
         // compiled passes for large states (the compile is amortised over many
-        // sweeps of the state), interpreted register tiles otherwise
+        // sweeps of the state)
         const bool jit = (k == 12 || k == 13) && !(flags & QF_EXEC_FLAG_NO_JIT) &&
                          ((flags & QF_EXEC_FLAG_JIT) || sv->n >= kJitMinQubits) && jit_available();
         if (jit) return run_plan_jit(sv, plan, 3);
@@ -830,6 +830,7 @@ int run_plan_dual(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_slot_su
     if (plan.passes.empty()) return QF_OK;
     if (psi->dtype != lambda->dtype || psi->n != lambda->n)
         return fail(QF_ERR_INCOMPATIBLE_DEVICE_STATE, "device states must have equal dimensions and dtype");
+    if (plan.vm) return run_plan_vm_dual(psi, lambda, plan, d_slot_sums);
     if (psi->dtype == QF_C64 && !(flags & QF_EXEC_FLAG_SMEM_TILES) && !(flags & QF_EXEC_FLAG_NO_JIT) &&
         ((flags & QF_EXEC_FLAG_JIT) || psi->n >= kJitMinQubits) && jit_available())
         return run_plan_jit_dual(psi, lambda, plan, d_slot_sums);
@@ -844,7 +845,7 @@ int reduce_slots(qf_ctx *ctx, const double *partials, uint32_t stride, uint32_t 
 }
 
 // Bound gate list on a resident state: unfused sweeps or tile passes.
-int execute_gates(qf_sv *sv, const std::vector<BGate> &gates, const qf_exec_opts *opts) {
+int execute_gates(qf_sv *sv, const std::vector<BGate> &gates, const qf_exec_opts *opts, bool resident) {
     const int mode = opts ? opts->mode : QF_EXEC_AUTO;
     if (mode == QF_EXEC_UNFUSED) {
         for (const BGate &g : gates) {
@@ -856,15 +857,15 @@ int execute_gates(qf_sv *sv, const std::vector<BGate> &gates, const qf_exec_opts
     if (mode != QF_EXEC_AUTO && mode != QF_EXEC_FUSED)
         return fail(QF_ERR_INVALID_ARGUMENT, "unknown execution mode %d", mode);
     PlanOpts po;
-    QF_TRY(plan_opts_for(sv->n, sv->dtype, opts, po));
+    QF_TRY(plan_opts_for(sv->n, sv->dtype, opts, resident, po));
     Plan plan;
     QF_TRY(plan_passes(sv->n, gates, po, plan));
     return run_plan(sv, plan, opts ? opts->flags : 0);
 }
 
 // Forward-sweep planning options from a caller's qf_exec_opts.
-int plan_opts_for(uint32_t n, int dtype, const qf_exec_opts *opts, PlanOpts &po) {
-    forward_tiling(n, dtype, opts ? opts->tile_qubits : 0, opts ? opts->flags : 0, &po.tile_qubits, &po.low_qubits);
+int plan_opts_for(uint32_t n, int dtype, const qf_exec_opts *opts, bool resident, PlanOpts &po) {
+    sweep_tiling(n, dtype, opts, false, resident, po);
     po.search = !(opts && (opts->flags & QF_EXEC_FLAG_PLAN_FIRST_COME));
     const int kb = opts ? opts->block_qubits : 0;
     if (kb < 0 || kb > kMaxBlockQubits)
