@@ -85,6 +85,40 @@ struct VmSink {
     virtual int launch(const VmHead &h, const VmRec *recs) = 0;
 };
 
+// ---- noisy shots: one CTA per trajectory (vmtraj.cu) -------------------------
+// A circuit with channels and measurements as runs of random decisions with
+// unitary record streams between them.
+enum TrajKind : uint8_t { TR_AD, TR_PD, TR_TH, TR_DEP, TR_MEAS };
+struct TrajStep {
+    uint8_t kind;
+    uint8_t pos;    // the qubit in the run's layout: register bit, or 4 + thread bit
+    uint8_t sd;     // state-dependent steps (all but TR_DEP): their number in the run
+    uint8_t later;  // a state-dependent step on the same qubit follows in the run
+    uint32_t cbit;
+    double p, gu;                // probability, gamma or gamma_down; gamma_up
+    double sp, s1p, su, s1u;     // square roots of p, 1 - p, gu, 1 - gu
+};
+struct TrajRun {
+    uint32_t rec_begin, n_recs;    // the unitary part before the decisions
+    uint32_t step_begin, n_steps;
+    uint32_t n_sd;                 // at most one per qubit, the first R of them on register bits 0, 1, ...
+    uint32_t terminal;             // measurements of distinct qubits with nothing after them
+};
+struct TrajProgram {
+    int R = 4, W = 3;
+    uint32_t n = 0;
+    uint64_t lcol[kVmMaxThreadBits] = {0}, lreg[4] = {0};  // state address bits of the layout at the start
+    std::vector<VmRec> recs;
+    std::vector<TrajRun> runs;
+    std::vector<TrajStep> steps;
+};
+constexpr uint32_t kTrajMaxQubits = 12;
+// *ok = false: a circuit the program form does not cover (feed-forward, invalid
+// operations).
+int vm_lower_trajectories(uint32_t n, const qf_op *ops, uint64_t n_ops, TrajProgram &out, bool *ok);
+int run_trajectories_vm(qf_sv *init, const TrajProgram &prog, uint64_t shots, const uint64_t *starts, double tie_eps,
+                        uint64_t *outcomes, uint64_t *n_ties);
+
 // Register and warp bits of a tile of k bits.
 void vm_shape(int k, int dtype, bool dual, int *R, int *W);
 // The widest tile the passes take, and the one they use when the caller names none.

@@ -279,12 +279,12 @@ struct Scheduler {
         }
         return S;
     }
-    bool run(Sched &out) {
+    bool run(Sched &out, const Layout *start) {
         const uint32_t low = (1u << std::min(low_bits(dtype), ps.k)) - 1u;
         const uint32_t every = (1u << ps.K) - 1u;
         // small tiles: registers must leave the lanes some bits
         const uint32_t first = ps.K - __builtin_popcount(low) >= ps.R ? every & ~low : every;
-        out.layouts.push_back(make_layout(ps, choose(first), true, dtype));
+        out.layouts.push_back(start ? *start : make_layout(ps, choose(first), true, dtype));
         uint32_t regs = 0;
         auto set_regs = [&] {
             regs = 0;
@@ -351,13 +351,15 @@ SchedCache &sched_cache() {
 }
 constexpr size_t kSchedEntries = 4096;
 
-std::shared_ptr<const Sched> schedule(const Pass &p, const PassSlots &ps, uint32_t n, int dtype) {
+// The pass's schedule; start: the layout its amplitudes already have.
+std::shared_ptr<const Sched> schedule(const Pass &p, const PassSlots &ps, uint32_t n, int dtype, const Layout *start = nullptr) {
     std::string key;
     key.reserve(11 + 3 * p.gates.size());
     key.append(reinterpret_cast<const char *>(&p.resident), 8);
     key.push_back((char)n);
     key.push_back((char)(ps.R | (ps.NT << 3)));
-    key.push_back((char)dtype);
+    key.push_back((char)(dtype | (start ? 2 : 0)));
+    if (start) key.append(reinterpret_cast<const char *>(start), sizeof *start);
     for (const BGate &g : p.gates) {
         const char e[3] = {(char)class_of(g), (char)g.q0, (char)g.q1};
         key.append(e, 3);
@@ -368,7 +370,7 @@ std::shared_ptr<const Sched> schedule(const Pass &p, const PassSlots &ps, uint32
         if (it != sched_cache().entries.end()) return it->second;
     }
     auto s = std::make_shared<Sched>();
-    if (!Scheduler(p.gates, ps, dtype).run(*s)) return nullptr;
+    if (!Scheduler(p.gates, ps, dtype).run(*s, start)) return nullptr;
     std::lock_guard<std::mutex> lk(sched_cache().mu);
     if (sched_cache().entries.size() >= kSchedEntries) sched_cache().entries.clear();  // bound the host memory
     sched_cache().entries[key] = s;
@@ -903,12 +905,7 @@ struct Emitter {
             if (fn[s].reg != kNone) m |= 1u << s;
         return m;
     }
-    // everything symbolic onto the amplitudes (end of the plan)
-    void flush_all() {
-        while (!terms.empty()) {
-            apply_term(terms.back());
-            terms.pop_back();
-        }
+    void emit_sign_frame() {
         bool signs = false;
         for (uint32_t q = 0; q < 64; ++q) {
             const uint64_t later_q = q == 63 ? 0 : adj[q] & (~0ULL << (q + 1));
@@ -924,6 +921,14 @@ struct Emitter {
             zmask = 0;
         }
         if (signs) rec(VM_FLUSHS);
+    }
+    // everything symbolic onto the amplitudes (end of the plan)
+    void flush_all() {
+        while (!terms.empty()) {
+            apply_term(terms.back());
+            terms.pop_back();
+        }
+        emit_sign_frame();
         if (scale.is_one()) return;
         if (!tph && scale.value().imag() == 0.0) {
             VmRec &w = rec(VM_SCALE);
@@ -935,6 +940,53 @@ struct Emitter {
         flush_phase();
     }
 
+    // the schedule's gates and remaps; cut: as many launches as the records need
+    int emit_steps(const Sched &sc, bool cut) {
+        later.assign(64, 0);
+        for (const BGate &g : pass->gates) {
+            const GClass c = class_of(g);
+            if (c == G_DENSE || c == G_OVXY) ++later[g.q0];
+        }
+        bool z_open = false;
+        for (const Step &st : sc.steps) {
+            if (cut && (int)recs.size() + reserve() > kVmCapacity) {  // cut the launch; the next one loads the same registers
+                const uint32_t keep = reg_slots();
+                QF_TRY(close(false));
+                open(make_layout(*ps, keep, true, dtype), true);
+                z_open = false;
+            }
+            if (st.gate == kNone) {
+                emit_remap(sc.layouts[st.layout]);
+                z_open = false;
+                continue;
+            }
+            const BGate &g = pass->gates[st.gate];
+            const GClass c = class_of(g);
+            switch (c) {
+            case G_DENSE: emit_dense(g.q0, g.m); --later[g.q0]; break;
+            case G_DIAG: emit_diag(g.q0, g.m); break;
+            case G_ANTI: emit_anti(g.q0, g.m); break;
+            case G_CNOT: emit_cnot(g.q0, g.q1); break;
+            case G_CZ: toggle(g.q0, g.q1); break;
+            case G_SWAP: emit_swap(g.q0, g.q1); std::swap(later[g.q0], later[g.q1]); break;
+            case G_OVXY: emit_overlap_xy(g); --later[g.q0]; break;
+            case G_OVZ: emit_overlap_z(g, !z_open); break;
+            }
+            z_open = c == G_OVZ;
+            while (terms.size() > (size_t)kMaxTerms) {
+                apply_term(terms.front());
+                terms.erase(terms.begin());
+            }
+            // factors pulled out grow the stored amplitudes: bounded well inside float32's range
+            if (scale.abs() < 0x1p-40) {  // a power of two: exact
+                VmRec &w = rec(VM_SCALE);
+                put(w.w + 4, 0, 0x1p-40);
+                scale *= 0x1p40;
+            }
+        }
+        return QF_OK;
+    }
+
     int run(int R, int W) {
         for (size_t pi = 0; pi < plan.passes.size(); ++pi) {
             pass = &plan.passes[pi];
@@ -942,54 +994,59 @@ struct Emitter {
             ps = &slots;
             const auto sc = schedule(*pass, slots, plan.n, dtype);
             if (!sc) return fail(QF_ERR_INVALID_ARGUMENT, "register-tile pass could not be scheduled");
-            const auto &G = pass->gates;
-            later.assign(64, 0);
-            for (const BGate &g : G) {
-                const GClass c = class_of(g);
-                if (c == G_DENSE || c == G_OVXY) ++later[g.q0];
-            }
             open(sc->layouts[0], false);
-            bool z_open = false;
-            for (const Step &st : sc->steps) {
-                if ((int)recs.size() + reserve() > kVmCapacity) {  // cut the launch; the next one loads the same registers
-                    const uint32_t keep = reg_slots();
-                    QF_TRY(close(false));
-                    open(make_layout(*ps, keep, true, dtype), true);
-                    z_open = false;
-                }
-                if (st.gate == kNone) {
-                    emit_remap(sc->layouts[st.layout]);
-                    z_open = false;
-                    continue;
-                }
-                const BGate &g = G[st.gate];
-                const GClass c = class_of(g);
-                switch (c) {
-                case G_DENSE: emit_dense(g.q0, g.m); --later[g.q0]; break;
-                case G_DIAG: emit_diag(g.q0, g.m); break;
-                case G_ANTI: emit_anti(g.q0, g.m); break;
-                case G_CNOT: emit_cnot(g.q0, g.q1); break;
-                case G_CZ: toggle(g.q0, g.q1); break;
-                case G_SWAP: emit_swap(g.q0, g.q1); std::swap(later[g.q0], later[g.q1]); break;
-                case G_OVXY: emit_overlap_xy(g); --later[g.q0]; break;
-                case G_OVZ: emit_overlap_z(g, !z_open); break;
-                }
-                z_open = c == G_OVZ;
-                while (terms.size() > (size_t)kMaxTerms) {
-                    apply_term(terms.front());
-                    terms.erase(terms.begin());
-                }
-                // factors pulled out grow the stored amplitudes: bounded well inside float32's range
-                if (scale.abs() < 0x1p-40) {  // a power of two: exact
-                    VmRec &w = rec(VM_SCALE);
-                    put(w.w + 4, 0, 0x1p-40);
-                    scale *= 0x1p40;
-                }
-            }
+            QF_TRY(emit_steps(*sc, true));
             QF_TRY(close(pi + 1 == plan.passes.size()));
         }
         return QF_OK;
     }
+    // One unitary part of a trajectory program: from layout `from` to exactly
+    // layout `to`, everything symbolic applied except the scalar (trajectories
+    // carry unnormalised states, and a global phase means nothing to them).
+    int segment(const PassSlots &slots, const Pass &p, const Layout &from, const Layout &to) {
+        pass = &p;
+        ps = &slots;
+        set_layout(from);
+        if (!p.gates.empty()) {
+            const auto sc = schedule(p, slots, plan.n, dtype, &from);
+            if (!sc) return fail(QF_ERR_INVALID_ARGUMENT, "register-tile segment could not be scheduled");
+            QF_TRY(emit_steps(*sc, false));
+        }
+        later.assign(64, 0);
+        apply_terms(false);  // on thread bits
+        flush_phase_only();
+        emit_sign_frame();
+        if (!holds(to)) emit_remap(to);
+        apply_terms(true);
+        flush_phase_only();
+        scale = Scalar();
+        return QF_OK;
+    }
+    bool holds(const Layout &to) const {  // the amplitudes lie exactly as `to` has them
+        for (int s = 0; s < ps->K; ++s)
+            if (fn[s].k || fn[s].Q) return false;
+        for (int i = 0; i < ps->NT; ++i)
+            if (fn[(int)to.tslot[i]].T != 1u << i || fn[(int)to.tslot[i]].reg != kNone) return false;
+        for (int r = 0; r < ps->R; ++r)
+            if (fn[(int)to.rslot[r]].reg != r || fn[(int)to.rslot[r]].T) return false;
+        return true;
+    }
+    void apply_terms(bool all) {
+        for (size_t i = 0; i < terms.size();) {
+            Fn r;
+            if (!all && regs_of(terms[i].mask, &r)) {
+                ++i;
+                continue;
+            }
+            apply_term(terms[i]);
+            terms.erase(terms.begin() + (long)i);
+        }
+    }
+    void flush_phase_only() {
+        if (tph) rec(VM_FLUSHP);
+        tph = false;
+    }
+
     // The records that one more step and the close of the launch can add: every
     // term, the sign frame, flushes, two remaps of up to eight records, a few gates.
     int reserve() const {
@@ -1001,6 +1058,167 @@ struct Emitter {
 };
 
 }  // namespace
+
+// Decisions of a channel or measurement commute with gates on other qubits, so a
+// gate joins the unitary part before the open run unless the run already acts
+// on one of its qubits; a run holds one state-dependent step per qubit. Lists
+// that the other engine refuses are left to it and its error texts.
+int vm_lower_trajectories(uint32_t n, const qf_op *ops, uint64_t n_ops, TrajProgram &out, bool *ok) {
+    *ok = false;
+    out = TrajProgram();
+    out.n = n;
+    out.R = std::min(std::max((int)n, 6) - 5, 4);
+    out.W = std::max((int)n, 6) - 5 - out.R;
+    struct Part {
+        std::vector<qf_op> gates, steps;
+    };
+    std::vector<Part> parts(1);
+    uint64_t touched = 0, dependent = 0;
+    for (uint64_t k = 0; k < n_ops; ++k) {
+        const qf_op &o = ops[k];
+        const bool gate = o.kind == QF_OP_GATE || o.kind == QF_OP_CNOT || o.kind == QF_OP_CZ || o.kind == QF_OP_SWAP;
+        if (!gate && o.kind != QF_OP_CHANNEL && o.kind != QF_OP_MEASURE) return QF_OK;
+        if (o.q0 >= n) return QF_OK;
+        const bool decision = o.kind == QF_OP_CHANNEL || o.kind == QF_OP_MEASURE;
+        uint64_t m = 1ULL << o.q0;
+        if (o.kind == QF_OP_CNOT || o.kind == QF_OP_CZ || o.kind == QF_OP_SWAP) {
+            if (o.q1 >= n || o.q1 == o.q0) return QF_OK;
+            m |= 1ULL << o.q1;
+        }
+        const bool sd = decision && !(o.kind == QF_OP_CHANNEL && o.gate == QF_CHANNEL_DEPOLARIZING);
+        if (decision ? (sd && (dependent & m)) : (touched & m) != 0) {
+            parts.emplace_back();
+            touched = dependent = 0;
+        }
+        if (decision) {
+            parts.back().steps.push_back(o);
+            touched |= m;
+            if (sd) dependent |= m;
+        } else {
+            parts.back().gates.push_back(o);
+        }
+    }
+    // trailing measurements of distinct qubits make a run of their own
+    {
+        std::vector<qf_op> &s = parts.back().steps;
+        size_t t = s.size();
+        while (t > 0 && s[t - 1].kind == QF_OP_MEASURE) --t;
+        if (t > 0 && t < s.size()) {
+            Part last;
+            last.steps.assign(s.begin() + (long)t, s.end());
+            s.resize(t);
+            parts.push_back(std::move(last));
+        }
+    }
+    std::vector<std::vector<BGate>> bound(parts.size());
+    for (size_t i = 0; i < parts.size(); ++i)
+        QF_TRY(bind_ops(n, parts[i].gates.data(), parts[i].gates.size(), nullptr, 0, nullptr, 0, -1, 0.0, bound[i]));
+    while (!parts.empty() && parts.back().steps.empty()) parts.pop_back();  // gates that no decision follows
+    Plan plan;
+    plan.n = n;
+    struct NoSink : VmSink {
+        int launch(const VmHead &, const VmRec *) override { return QF_OK; }
+    } none;
+    Emitter e(plan, QF_C128, none);
+    Layout at;
+    for (size_t pi = 0; pi < parts.size(); ++pi) {
+        const std::vector<BGate> &gates = bound[pi];
+        Pass p;
+        p.resident = (1ULL << n) - 1;
+        if (!gates.empty()) {  // one-qubit runs merged
+            PlanOpts po;
+            po.tile_qubits = po.low_qubits = (int)n;
+            po.search = false;
+            po.vm = po.merge_any = true;
+            po.max_items = 1 << 30;
+            Plan merged;
+            QF_TRY(plan_passes(n, gates, po, merged));
+            for (const Pass &x : merged.passes) p.gates.insert(p.gates.end(), x.gates.begin(), x.gates.end());
+        }
+        const PassSlots slots(p, n, out.R, out.W);
+        // the run's layout
+        const std::vector<qf_op> &st = parts[pi].steps;
+        TrajRun r{};
+        r.terminal = pi + 1 == parts.size();
+        std::vector<int> order;  // state-dependent qubits in order
+        for (const qf_op &o : st) {
+            r.terminal = r.terminal && o.kind == QF_OP_MEASURE;
+            if (!(o.kind == QF_OP_CHANNEL && o.gate == QF_CHANNEL_DEPOLARIZING)) order.push_back((int)o.q0);
+        }
+        r.n_sd = (uint32_t)order.size();
+        uint32_t used = 0;
+        Layout to;
+        std::memset(&to, kNone, sizeof to);
+        for (int q : order) used |= 1u << q;
+        std::vector<int> all = order;
+        for (int s = slots.K - 1; s >= 0; --s)
+            if (!((used >> s) & 1u)) all.push_back(s);
+        if (r.terminal) {  // first measured on the highest thread bit, the last ones on registers
+            for (int i = 0; i < slots.NT; ++i) to.tslot[slots.NT - 1 - i] = (int8_t)all[i];
+            for (int i = 0; i < slots.R; ++i) to.rslot[slots.R - 1 - i] = (int8_t)all[slots.NT + i];
+        } else {  // the first state-dependent ones on register bits 0, 1, ...
+            for (int i = 0; i < slots.R; ++i) to.rslot[i] = (int8_t)all[i];
+            uint32_t rest = 0;
+            for (int i = slots.R; i < slots.K; ++i) rest |= 1u << all[i];
+            for (int s = 0, i = 0; s < slots.K; ++s)
+                if ((rest >> s) & 1u) to.tslot[i++] = (int8_t)s;
+        }
+        if (pi == 0) {
+            at = make_layout(slots, 0, true, QF_C128);
+            for (int i = 0; i < slots.NT; ++i) out.lcol[i] = slots.address_bit(at.tslot[i]);
+            for (int i = 0; i < slots.R; ++i) out.lreg[i] = slots.address_bit(at.rslot[i]);
+        }
+        r.rec_begin = (uint32_t)e.recs.size();
+        QF_TRY(e.segment(slots, p, at, to));
+        r.n_recs = (uint32_t)e.recs.size() - r.rec_begin;
+        at = to;
+        uint8_t pos[64];
+        for (int i = 0; i < slots.NT; ++i) pos[(int)to.tslot[i]] = (uint8_t)(4 + i);
+        for (int i = 0; i < slots.R; ++i) pos[(int)to.rslot[i]] = (uint8_t)i;
+        r.step_begin = (uint32_t)out.steps.size();
+        r.n_steps = (uint32_t)st.size();
+        uint32_t n_sd = 0;
+        for (size_t i = 0; i < st.size(); ++i) {
+            const qf_op &o = st[i];
+            TrajStep t{};
+            t.pos = pos[o.q0];
+            t.cbit = o.param;
+            t.kind = TR_MEAS;
+            if (o.kind == QF_OP_CHANNEL) {
+                t.p = o.theta;
+                if (!std::isfinite(t.p) || t.p < 0.0 || t.p > 1.0) return QF_OK;
+                if (o.gate == QF_CHANNEL_THERMAL_DAMPING) {
+                    const double beta = qf_op_aux(&o);
+                    if (!std::isfinite(beta) || beta < 0.0) return QF_OK;
+                    t.gu = t.p * std::exp(-beta);  // NoiseChannel::thermal_rates (src/lib.rs:1611-1626)
+                }
+                switch (o.gate) {
+                case QF_CHANNEL_DEPOLARIZING: t.kind = TR_DEP; break;
+                case QF_CHANNEL_AMPLITUDE_DAMPING: t.kind = TR_AD; break;
+                case QF_CHANNEL_PHASE_DAMPING: t.kind = TR_PD; break;
+                case QF_CHANNEL_THERMAL_DAMPING: t.kind = TR_TH; break;
+                default: return QF_OK;
+                }
+                t.sp = std::sqrt(t.p);
+                t.s1p = std::sqrt(1.0 - t.p);
+                t.su = std::sqrt(t.gu);
+                t.s1u = std::sqrt(1.0 - t.gu);
+            }
+            if (t.kind == TR_DEP) {
+                for (size_t j = i + 1; j < st.size(); ++j)
+                    if (st[j].q0 == o.q0 && !(st[j].kind == QF_OP_CHANNEL && st[j].gate == QF_CHANNEL_DEPOLARIZING)) t.later = 1;
+            } else {
+                t.sd = (uint8_t)n_sd++;
+            }
+            out.steps.push_back(t);
+        }
+        out.runs.push_back(r);
+    }
+    out.recs = std::move(e.recs);
+    out.recs.emplace_back();  // the interpreter reads one head ahead
+    *ok = !out.runs.empty();
+    return QF_OK;
+}
 
 int vm_lower(const Plan &plan, int dtype, int R, int W, VmSink &sink) { return Emitter(plan, dtype, sink).run(R, W); }
 
