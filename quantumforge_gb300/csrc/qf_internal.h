@@ -331,6 +331,10 @@ int jit_check_compile(const Plan &plan, int wb, std::string *source, std::string
 // shared-memory kernel).
 int run_plan_dual(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_slot_sums, int flags = 0);
 int run_plan_dual_smem(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_slot_sums);
+// The same passes in groups of ops that share one assignment of amplitudes to
+// threads (complex64; dualpass.cu); plans it does not cover run on the
+// interpreter above.
+int run_plan_dual_groups(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_slot_sums);
 // Compiled backward passes; falls back to run_plan_dual_smem for plans the
 // compiled layout does not cover.
 int run_plan_jit_dual(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_slot_sums);

@@ -834,6 +834,7 @@ int run_plan_dual(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_slot_su
     if (psi->dtype == QF_C64 && !(flags & QF_EXEC_FLAG_SMEM_TILES) && !(flags & QF_EXEC_FLAG_NO_JIT) &&
         ((flags & QF_EXEC_FLAG_JIT) || psi->n >= kJitMinQubits) && jit_available())
         return run_plan_jit_dual(psi, lambda, plan, d_slot_sums);
+    if (psi->dtype == QF_C64 && !(flags & QF_EXEC_FLAG_SMEM_TILES)) return run_plan_dual_groups(psi, lambda, plan, d_slot_sums);
     return run_plan_dual_smem(psi, lambda, plan, d_slot_sums);
 }
 
