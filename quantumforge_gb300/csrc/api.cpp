@@ -1460,7 +1460,18 @@ int run_density_steps(qf_sv *sv, uint32_t n, const std::vector<DmStep> &steps, c
         }
         size_t e = i;
         while (e < steps.size() && steps[e].channel) ++e;
-        if (n < 3 || sv->dtype != QF_C64) {
+        if (sv->dtype != QF_C64) {
+            std::vector<uint32_t> qs;
+            std::vector<std::array<double, 6>> cf;
+            for (; i < e; ++i) {
+                qs.push_back(steps[i].q);
+                cf.emplace_back();
+                std::copy(steps[i].coef, steps[i].coef + 6, cf.back().begin());
+            }
+            QF_TRY(dm_channel_run(sv, n, qs.data(), reinterpret_cast<const double(*)[6]>(cf.data()), qs.size()));
+            continue;
+        }
+        if (n < 3) {
             for (; i < e; ++i) QF_TRY(dm_channel(sv, n, steps[i].q, steps[i].coef));
             continue;
         }

@@ -148,8 +148,7 @@ struct ChannelTile {
     uint64_t hi_bits[kMaxTileChannels * 2];
     uint32_t n_ch;
     uint8_t lc[kMaxTileChannels], lr[kMaxTileChannels], shape[kMaxTileChannels];
-    double coef[kMaxTileChannels][6];
-    float coef_f[kMaxTileChannels][6];  // the same in f32: no f64 -> f32 conversion per tile for complex64
+    float coef_f[kMaxTileChannels][6];
     // complex64 paired rounds (k = 12): per round its channels (0xFF: none),
     // the tile bits of the thread's eight index bits, the swizzled offsets of
     // its 16 entries and whether entries i, i + 1 share a 16-byte slot
@@ -160,12 +159,10 @@ struct ChannelTile {
     uint32_t n_rounds;
 };
 
-template <typename C>
-__global__ void __launch_bounds__(256) k_dm_channel_tile(C *__restrict__ v, uint64_t n_tiles, const ChannelTile ct) {
-    using R = typename Real<C>::T;
+__global__ void __launch_bounds__(256) k_dm_channel_tile(float2 *__restrict__ v, uint64_t n_tiles, const ChannelTile ct) {
     extern __shared__ __align__(16) unsigned char dm_smem[];
-    C *s = reinterpret_cast<C *>(dm_smem);
-    uint64_t *hi_off = reinterpret_cast<uint64_t *>(dm_smem + (sizeof(C) << ct.k));
+    float2 *s = reinterpret_cast<float2 *>(dm_smem);
+    uint64_t *hi_off = reinterpret_cast<uint64_t *>(dm_smem + (sizeof(float2) << ct.k));
     const uint32_t T = 1u << ct.k;
     for (uint32_t h = threadIdx.x; h < (1u << ct.n_hi); h += blockDim.x) {
         uint64_t off = 0;
@@ -176,35 +173,25 @@ __global__ void __launch_bounds__(256) k_dm_channel_tile(C *__restrict__ v, uint
     __syncthreads();
     for (uint64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
         const uint64_t base = deposit(t, ct.outer_mask);
-        if (sizeof(C) == 8) {  // complex64: 16-byte accesses (2 amplitudes of a 32-amplitude run), all in flight
 #pragma unroll 8
-            for (uint32_t w = threadIdx.x; w < (T >> 1); w += blockDim.x) {
-                const uint32_t j = w << 1;
-                *reinterpret_cast<float4 *>(s + j) = *reinterpret_cast<const float4 *>(v + (base | hi_off[j >> 5] | (j & 31u)));
-            }
-        } else {
-            for (uint32_t j = threadIdx.x; j < T; j += blockDim.x) s[j] = v[base | hi_off[j >> 5] | (j & 31u)];
+        for (uint32_t w = threadIdx.x; w < (T >> 1); w += blockDim.x) {  // 16-byte accesses (2 amplitudes of a 32-amplitude run), all in flight
+            const uint32_t j = w << 1;
+            *reinterpret_cast<float4 *>(s + j) = *reinterpret_cast<const float4 *>(v + (base | hi_off[j >> 5] | (j & 31u)));
         }
         __syncthreads();
         for (uint32_t c = 0; c < ct.n_ch; ++c) {
             const uint32_t lc = ct.lc[c], lr = ct.lr[c], lo = min(lc, lr), hi = max(lc, lr);
             const uint32_t cm = 1u << lc, rm = 1u << lr;
-            R a, b, cc, d, e, f;
-            if (sizeof(R) == 4) {
-                a = (R)ct.coef_f[c][0], b = (R)ct.coef_f[c][1], cc = (R)ct.coef_f[c][2], d = (R)ct.coef_f[c][3];
-                e = (R)ct.coef_f[c][4], f = (R)ct.coef_f[c][5];
-            } else {
-                a = (R)ct.coef[c][0], b = (R)ct.coef[c][1], cc = (R)ct.coef[c][2], d = (R)ct.coef[c][3];
-                e = (R)ct.coef[c][4], f = (R)ct.coef[c][5];
-            }
+            const float a = ct.coef_f[c][0], b = ct.coef_f[c][1], cc = ct.coef_f[c][2], d = ct.coef_f[c][3], e = ct.coef_f[c][4],
+                        f = ct.coef_f[c][5];
             const int shape = ct.shape[c];
             for (uint32_t g = threadIdx.x; g < (T >> 2); g += blockDim.x) {
                 uint32_t i = g;
                 i = ((i >> lo) << (lo + 1)) | (i & ((1u << lo) - 1u));
                 i = ((i >> hi) << (hi + 1)) | (i & ((1u << hi) - 1u));
-                const C x01 = s[i | cm], x10 = s[i | rm];
+                const float2 x01 = s[i | cm], x10 = s[i | rm];
                 if (shape != 2) {
-                    const C x00 = s[i], x11 = s[i | rm | cm];
+                    const float2 x00 = s[i], x11 = s[i | rm | cm];
                     s[i] = mk(a * x00.x + b * x11.x, a * x00.y + b * x11.y);
                     s[i | rm | cm] = mk(cc * x00.x + d * x11.x, cc * x00.y + d * x11.y);
                 }
@@ -213,14 +200,10 @@ __global__ void __launch_bounds__(256) k_dm_channel_tile(C *__restrict__ v, uint
             }
             __syncthreads();
         }
-        if (sizeof(C) == 8) {
 #pragma unroll 8
-            for (uint32_t w = threadIdx.x; w < (T >> 1); w += blockDim.x) {
-                const uint32_t j = w << 1;
-                *reinterpret_cast<float4 *>(v + (base | hi_off[j >> 5] | (j & 31u))) = *reinterpret_cast<const float4 *>(s + j);
-            }
-        } else {
-            for (uint32_t j = threadIdx.x; j < T; j += blockDim.x) v[base | hi_off[j >> 5] | (j & 31u)] = s[j];
+        for (uint32_t w = threadIdx.x; w < (T >> 1); w += blockDim.x) {
+            const uint32_t j = w << 1;
+            *reinterpret_cast<float4 *>(v + (base | hi_off[j >> 5] | (j & 31u))) = *reinterpret_cast<const float4 *>(s + j);
         }
         __syncthreads();
     }
@@ -367,7 +350,7 @@ int dm_channel(qf_sv *sv, uint32_t n, uint32_t q, const double coef[6]) {
 int dm_channels_fused(qf_sv *sv, uint32_t n, const uint32_t *qs, const double (*coefs)[6], uint32_t count) {
     qf_ctx *ctx = sv->ctx;
     if (count == 0) return QF_OK;
-    if (count > (uint32_t)kMaxTileChannels || 2 * n < 5) return fail(QF_ERR_INVALID_ARGUMENT, "channel group too large");
+    if (sv->dtype != QF_C64 || count > (uint32_t)kMaxTileChannels || 2 * n < 5) return fail(QF_ERR_INVALID_ARGUMENT, "channel group too large");
     // the kernel moves complex64 entries two at a time (16-byte accesses): the
     // tile's low five bits are column bits 0..4 and the matrix is 16-byte aligned
     if (reinterpret_cast<uintptr_t>(sv->d) % 16)
@@ -398,12 +381,11 @@ int dm_channels_fused(qf_sv *sv, uint32_t n, const uint32_t *qs, const double (*
         const double *k = coefs[c];
         ct.shape[c] = (k[0] == 1.0 && k[1] == 0.0 && k[2] == 0.0 && k[3] == 1.0) ? 2 : 0;
         for (int j = 0; j < 6; ++j) {
-            ct.coef[c][j] = k[j];
             ct.coef_f[c][j] = (float)k[j];
         }
     }
     const uint64_t n_tiles = 1ULL << (2 * n - ct.k);
-    const bool pairs = sv->dtype == QF_C64 && ct.k == 12 && 2 * n - ct.k <= 24;
+    const bool pairs = ct.k == 12 && 2 * n - ct.k <= 24;
     if (pairs) {
         // channels in pairs (they act on disjoint bits and commute); a channel
         // whose column bit is tile bit 0 goes first in its round, so the
@@ -476,14 +458,10 @@ int dm_channels_fused(qf_sv *sv, uint32_t n, const uint32_t *qs, const double (*
         QF_CUDA(cudaFuncSetAttribute(k_dm_channel_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         QF_TRY(grid_of((const void *)k_dm_channel_pairs, &grid));
         k_dm_channel_pairs<<<grid, 256, smem, ctx->stream>>>(static_cast<float2 *>(sv->d), n_tiles, ct);
-    } else if (sv->dtype == QF_C64) {
-        QF_CUDA(cudaFuncSetAttribute(k_dm_channel_tile<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        QF_TRY(grid_of((const void *)k_dm_channel_tile<float2>, &grid));
-        k_dm_channel_tile<float2><<<grid, 256, smem, ctx->stream>>>(static_cast<float2 *>(sv->d), n_tiles, ct);
     } else {
-        QF_CUDA(cudaFuncSetAttribute(k_dm_channel_tile<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        QF_TRY(grid_of((const void *)k_dm_channel_tile<double2>, &grid));
-        k_dm_channel_tile<double2><<<grid, 256, smem, ctx->stream>>>(static_cast<double2 *>(sv->d), n_tiles, ct);
+        QF_CUDA(cudaFuncSetAttribute(k_dm_channel_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        QF_TRY(grid_of((const void *)k_dm_channel_tile, &grid));
+        k_dm_channel_tile<<<grid, 256, smem, ctx->stream>>>(static_cast<float2 *>(sv->d), n_tiles, ct);
     }
     QF_CUDA(cudaGetLastError());
     return QF_OK;
