@@ -1080,56 +1080,112 @@ __global__ void k_marginal(const C *__restrict__ a, uint32_t n, const uint32_t *
     }
 }
 
-// level k (2^k entries at offset 2^k - 1) from level k+1
-__global__ void k_tree_level(double *tree, uint32_t k) {
-    const uint64_t cnt = 1ULL << k;
-    double *dst = tree + (cnt - 1), *src = tree + (2 * cnt - 1);
-    for (uint64_t b = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; b < cnt; b += (uint64_t)gridDim.x * blockDim.x)
-        dst[b] = src[b] + src[b | cnt];
-}
-
-__device__ __forceinline__ uint64_t gf2_apply(const uint64_t *cols, uint64_t x) {
-    uint64_t y = 0;
-    while (x) {
-        const int c = __ffsll((long long)x) - 1;
-        y ^= cols[c];
-        x &= x - 1;
+// Levels k1 - 1 .. k1 - F of the tree (level k: 2^k entries at offset 2^k - 1)
+// from level k1: an entry of level k adds the two of level k + 1 that differ in
+// their top bit. A CTA folds the entries of `runs` consecutive low indices (64
+// bytes per access) through all F levels in shared memory: 20 levels took 20
+// launches of 4.1 us, here two of 16 and 11. The launch that ends at the root also fills the
+// lanes' table (k_shots) from its other CTAs.
+constexpr uint32_t kFoldLevels = 10, kFoldRunBits = 3, kFoldRuns = 1u << kFoldRunBits;
+__global__ void __launch_bounds__(256) k_tree_fold(double *tree, uint32_t k1, uint32_t levels, uint32_t n_fold,
+                                                   const uint64_t *__restrict__ jump, uint64_t *__restrict__ lanes) {
+    extern __shared__ double fold[];
+    if (blockIdx.x >= n_fold) {  // column c of the matrix that skips l shots, l = 0..31
+        uint64_t *mat = reinterpret_cast<uint64_t *>(fold);
+        for (uint32_t e = threadIdx.x; e < 5 * 64; e += blockDim.x) mat[e] = jump[e];
+        __syncthreads();
+        const uint32_t i = (blockIdx.x - n_fold) * blockDim.x + threadIdx.x, c = i >> 5, l = i & 31u;
+        uint64_t x = 1ULL << c;
+        for (uint32_t j = 0; j < 5; ++j)
+            if ((l >> j) & 1u) {
+                uint64_t y = 0;
+                for (uint64_t r = x; r; r &= r - 1) y ^= mat[64 * j + __ffsll((long long)r) - 1];
+                x = y;
+            }
+        lanes[i] = x;
+        return;
     }
-    return y;
+    const uint64_t low = 1ULL << (k1 - levels);  // low indices
+    const uint32_t sh = low < kFoldRuns ? k1 - levels : kFoldRunBits, runs = 1u << sh;
+    const uint64_t b0 = (uint64_t)blockIdx.x * runs;
+    const double *src = tree + ((1ULL << k1) - 1);
+    for (uint32_t i = threadIdx.x; i < (runs << levels); i += blockDim.x) fold[i] = src[(uint64_t)(i >> sh) * low + b0 + (i & (runs - 1))];
+    for (uint32_t f = levels; f-- > 0;) {
+        __syncthreads();
+        const uint32_t half = runs << f;
+        double *dst = tree + ((low << f) - 1);
+        for (uint32_t i = threadIdx.x; i < half; i += blockDim.x) {
+            const double v = fold[i] + fold[i + half];
+            fold[i] = v;
+            dst[(uint64_t)(i >> sh) * low + b0 + (i & (runs - 1))] = v;
+        }
+    }
 }
 
+// x > 0 as float32 by its bits (truncated; 0 below the float32 range), off the FP64 pipe
+__device__ __forceinline__ float float_of(double x) {
+    const int hi = __double2hiint(x);
+    return hi < (897 << 20) ? 0.f : __uint_as_float(((uint32_t)(hi - (896 << 20)) << 3) | ((uint32_t)__double2loint(x) >> 29));
+}
+
+// A division, three products and two comparisons per measurement in FP64 bound
+// this kernel (100k shots of 20 qubits: 129 us, a third of it the generator's
+// jumps, 32 matrix columns per set bit of the shot's number; 16 us now). A float32 quotient
+// now decides every outcome that it can (off by less than 2^-20, and ties cannot
+// be closer than `margin`); only the others divide. The branch's mass D takes one
+// addition: D p = J1 and D (1 - p) = D - J1. Shots s0..s0 + 31 of a warp share
+// the jump to s0, one column per lane, and the last five bits come from a table.
 __global__ void k_shots(const double *__restrict__ tree, uint32_t m, const uint32_t *__restrict__ cbits, uint64_t shots,
-                        uint64_t seed_state, const uint64_t *__restrict__ jump, const uint64_t *__restrict__ starts,
-                        int normalize, double tie_eps, uint64_t *__restrict__ outcomes, unsigned long long *__restrict__ ties,
-                        int *__restrict__ err) {
-    for (uint64_t s = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; s < shots; s += (uint64_t)gridDim.x * blockDim.x) {
+                        uint64_t seed_state, const uint64_t *__restrict__ jump, uint32_t n_jump, const uint64_t *__restrict__ lanes,
+                        const uint64_t *__restrict__ starts, int normalize, double tie_eps, float margin,
+                        uint64_t *__restrict__ outcomes, unsigned long long *__restrict__ ties, int *__restrict__ err) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint64_t s0 = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) - lane; s0 < shots; s0 += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t s = s0 + lane;
         uint64_t x = seed_state;
         if (starts) {  // the shot's generator state given (shots of one branch of a feed-forward circuit)
-            x = starts[s];
+            x = s < shots ? starts[s] : 1;
         } else {
-            for (int j = 0; j < 64; ++j)
-                if ((s >> j) & 1ULL) x = gf2_apply(jump + 64 * j, x);
+            for (uint32_t j = 5; j < n_jump; ++j)
+                if ((s0 >> j) & 1ULL) {
+                    const uint64_t y = (((x >> lane) & 1ULL) ? jump[64 * j + lane] : 0) ^
+                                       (((x >> (lane + 32)) & 1ULL) ? jump[64 * j + 32 + lane] : 0);
+                    x = (uint64_t)__reduce_xor_sync(0xffffffffu, (uint32_t)(y >> 32)) << 32 |
+                        __reduce_xor_sync(0xffffffffu, (uint32_t)y);
+                }
+            uint64_t y = 0;
+            for (uint64_t r = x; r; r &= r - 1) y ^= lanes[32 * (__ffsll((long long)r) - 1) + lane];
+            x = y;
         }
+        if (s >= shots) continue;
         uint64_t b = 0, reg = 0;
         double D = normalize ? tree[0] : 1.0;  // complex64: probabilities relative to the state's own norm
         unsigned long long nt = 0;
         for (uint32_t k = 0; k < m; ++k) {
             const double J1 = tree[((1ULL << (k + 1)) - 1) + (b | (1ULL << k))];
-            double p = J1 / D;
-            if (p < 0.0) p = 0.0;
-            if (p > 1.0) p = 1.0;
             x ^= x << 13;
             x ^= x >> 7;
             x ^= x << 17;
-            const double u = (double)(x >> 11) * (1.0 / 9007199254740992.0);
-            const int o = u < p ? 1 : 0;
-            if (fabs(u - p) < tie_eps) ++nt;
-            const double prob = o ? p : 1.0 - p;
-            if (prob <= 2.220446049250313e-16) {
-                atomicOr(err, 1);
-                break;
+            const float pf = __fdividef(float_of(J1), float_of(D)), uf = (float)(uint32_t)(x >> 40) * 5.9604644775390625e-8f;
+            int o = uf < pf ? 1 : 0;
+            const bool in_range = (uint32_t)__double2hiint(J1) < (1143u << 20) &&
+                                  (uint32_t)(__double2hiint(D) - (961 << 20)) < ((1143u - 961u) << 20);
+            if (!(in_range && fabsf(uf - pf) > margin)) {
+                double p = J1 / D;
+                if (p < 0.0) p = 0.0;
+                if (p > 1.0) p = 1.0;
+                const double u = (double)(x >> 11) * (1.0 / 9007199254740992.0);
+                o = u < p ? 1 : 0;
+                if (fabs(u - p) < tie_eps) ++nt;
+                const double prob = o ? p : 1.0 - p;
+                if (prob <= 2.220446049250313e-16) {
+                    atomicOr(err, 1);
+                    break;
+                }
             }
-            D *= prob;
+            // D p, with p at most 1 (positive doubles order as integers)
+            if (!o) D -= J1;
+            else if (__double_as_longlong(J1) < __double_as_longlong(D)) D = J1;
             b |= (uint64_t)o << k;
             reg = (reg & ~(1ULL << cbits[k])) | ((uint64_t)o << cbits[k]);
         }
@@ -1158,10 +1214,10 @@ int sample_shots(qf_sv *sv, const uint32_t *qubits, const uint32_t *cbits, uint3
     }
     const uint64_t valid = n >= 64 ? ~0ULL : ((1ULL << n) - 1);
     const uint64_t rest = valid & ~seen;
-    // workspace: tree (2^(m+1) doubles) | outcomes (shots u64) | jump (64*64 u64) | mq | cb | ties | err | starts
+    // workspace: tree (2^(m+1) doubles) | outcomes (shots u64) | jump (64*64 u64) and lanes (32*64) | mq | cb | ties | err | starts
     const size_t tree_b = sizeof(double) * ((2ULL << m));
     const size_t out_b = sizeof(uint64_t) * shots;
-    const size_t jump_b = sizeof(uint64_t) * 64 * 64;
+    const size_t jump_b = sizeof(uint64_t) * (64 + 32) * 64;
     const size_t meta_b = 2 * sizeof(uint32_t) * 32 + 64;
     const size_t start_b = start_states ? sizeof(uint64_t) * shots : 0;
     QF_TRY(ensure_device(&ctx->ws_tree, &ctx->ws_tree_bytes, tree_b + out_b + jump_b + meta_b + start_b));
@@ -1177,8 +1233,11 @@ int sample_shots(qf_sv *sv, const uint32_t *qubits, const uint32_t *cbits, uint3
     if (d_starts) QF_CUDA(cudaMemcpyAsync(d_starts, start_states, start_b, cudaMemcpyHostToDevice, ctx->stream));
 
     static thread_local uint64_t jump[64][64];
-    rng_jump_matrices(m, jump, 64);
-    QF_CUDA(cudaMemcpyAsync(d_jump, jump, jump_b, cudaMemcpyHostToDevice, ctx->stream));
+    uint32_t n_jump = 5;  // bits of a shot's number
+    while (n_jump < 64 && (shots - 1) >> n_jump) ++n_jump;
+    rng_jump_matrices(m, jump, (int)n_jump);
+    QF_CUDA(cudaMemcpyAsync(d_jump, jump, sizeof(jump[0]) * n_jump, cudaMemcpyHostToDevice, ctx->stream));
+    uint64_t *d_lanes = d_jump + 64 * 64;
     if (m) {
         QF_CUDA(cudaMemcpyAsync(d_mq, qubits, sizeof(uint32_t) * m, cudaMemcpyHostToDevice, ctx->stream));
         QF_CUDA(cudaMemcpyAsync(d_cb, cbits, sizeof(uint32_t) * m, cudaMemcpyHostToDevice, ctx->stream));
@@ -1193,10 +1252,16 @@ int sample_shots(qf_sv *sv, const uint32_t *qubits, const uint32_t *cbits, uint3
     else
         k_marginal<double2><<<grid, 256, 0, ctx->stream>>>(static_cast<double2 *>(sv->d), n, d_mq, m, rest, leaf);
     QF_CUDA(cudaGetLastError());
-    for (int k = (int)m - 1; k >= 0; --k) {
-        const uint64_t cnt = 1ULL << k;
-        k_tree_level<<<std::max(1, std::min<int>((int)((cnt + 255) / 256), ctx->sm_count * 8)), 256, 0, ctx->stream>>>(tree, (uint32_t)k);
+    static size_t dyn[64] = {0};
+    const int dev = ctx->device & 63;
+    if (!dyn[dev]) QF_TRY(allow_max_dynamic_smem(k_tree_fold, ctx, &dyn[dev]));
+    for (uint32_t k = m; k > 0;) {
+        const uint32_t levels = std::min(k, kFoldLevels);
+        const uint64_t low = 1ULL << (k - levels), runs = std::min<uint64_t>(low, kFoldRuns);
+        const uint32_t n_fold = (uint32_t)(low / runs), extra = levels == k ? 64 * 32 / 256 : 0;
+        k_tree_fold<<<n_fold + extra, 256, sizeof(double) * std::max<uint64_t>(runs << levels, 5 * 64), ctx->stream>>>(tree, k, levels, n_fold, d_jump, d_lanes);
         QF_CUDA(cudaGetLastError());
+        k -= levels;
     }
     const uint64_t seed_state = [&] {
         uint64_t z = seed + 0x9E3779B97F4A7C15ULL;
@@ -1206,8 +1271,10 @@ int sample_shots(qf_sv *sv, const uint32_t *qubits, const uint32_t *cbits, uint3
         return z == 0 ? 0x9E3779B97F4A7C15ULL : z;
     }();
     const int sgrid = std::max(1, std::min<int>((int)((shots + 127) / 128), ctx->sm_count * 16));
-    k_shots<<<sgrid, 128, 0, ctx->stream>>>(tree, m, d_cb, shots, seed_state, d_jump, d_starts, sv->dtype == QF_C64 ? 1 : 0,
-                                            tie_eps, d_out, d_ties, d_err);
+    // a margin of 2^-17 covers the float32 quotient's error eight times
+    const float margin = (float)(7.62939453125e-6 + 1.0001 * std::fabs(tie_eps));
+    k_shots<<<sgrid, 128, 0, ctx->stream>>>(tree, m, d_cb, shots, seed_state, d_jump, n_jump, d_lanes, d_starts,
+                                            sv->dtype == QF_C64 ? 1 : 0, tie_eps, margin, d_out, d_ties, d_err);
     QF_CUDA(cudaGetLastError());
     if (outcomes_host)
         QF_CUDA(cudaMemcpyAsync(outcomes_host, d_out, out_b, cudaMemcpyDeviceToHost, ctx->stream));
