@@ -1,5 +1,5 @@
 // qaoa.cu — batched QAOA MaxCut: cost and adjoint gradient for many
-// instances of uneven qubit counts in one persistent launch.
+// instances of uneven qubit counts.
 //
 // The circuit is algorithms::qaoa_maxcut (src/algorithms.rs:110-137): H on
 // every qubit, then per layer CNOT(u,v)·Rz(2γw)·CNOT(u,v) for every edge and
@@ -10,8 +10,10 @@
 // C(x) (unit weights) or computed from it. The mixer is exp(-iβ X) on every
 // qubit.
 //
-// Each CTA takes instances from an atomic counter (no waiting on other CTAs)
-// and runs the whole forward sweep, the costate λ = C ψ and the reverse sweep
+// Instances of up to 12 qubits run one CTA each in shared memory, larger ones
+// in tile passes over all instances of a qubit count (both below). With a tile
+// width given, each CTA takes instances from an atomic counter (no waiting on
+// other CTAs) and runs the whole forward sweep, the costate λ = C ψ and the reverse sweep
 // for its instance, with ψ, λ and a uint8 table of C(x) in a per-instance
 // arena (L2/HBM). Gates run in shared-memory tiles of 2^k amplitudes (k per
 // instance, autotuned per qubit count); inside a tile, mixer gates are applied
@@ -330,6 +332,174 @@ __global__ void __launch_bounds__(kQThreads)
     }
 }
 
+// ---- instances of up to 12 qubits ---------------------------------------------
+// psi, lambda, the cut values and the phase tables of all layers stay in the
+// CTA's shared memory from H|0> to the gradients. The per-instance kernel above
+// took 1166 us for 12 qubits and 4 layers: its second pass walked 128 tiles of 32
+// amplitudes, and each layer computed its angles' sines again in FP64 by every
+// thread (65 us here, for 93 instances). Its float32 operations are kept, and so are their sums: a
+// thread's products of one group of 2^NB amplitudes add up in float32, everything
+// else in double. Rounds: bits 0..3, 4..7, 8..9, then 10..11 (the second pass).
+struct SmallLayout {
+    uint32_t tl, cost, phase, mixer, emask, red, total;  // byte offsets behind psi
+};
+__host__ __device__ inline SmallLayout small_layout(uint32_t n, uint32_t p, uint32_t edges) {
+    SmallLayout L;
+    uint32_t off = 8u << n;
+    auto take = [&](uint32_t bytes) {
+        const uint32_t at = off;
+        off += (bytes + 15) / 16 * 16;
+        return at;
+    };
+    L.tl = take(8u << n);
+    L.cost = take(1u << n);
+    L.phase = take(8 * p * (edges + 1));
+    L.mixer = take(16 * p);
+    L.emask = take(4 * edges);
+    L.red = take(8 * 2 * 2 * kQThreads);
+    L.total = off;
+    return L;
+}
+__device__ __forceinline__ uint32_t small_phys(uint32_t j) { return j ^ ((j >> 4) & 15u); }
+
+// exp(-i beta X) on bits b0..b0+NB-1; ph: the cost phase first; DUAL: both states
+// and 2 Im<lambda|X_q|psi> (before the gate) into g
+template <bool DUAL, int NB>
+__device__ __forceinline__ void small_round(float2 *tp, float2 *tl, uint32_t n, uint32_t b0, float c, float s, double &g,
+                                            const float2 *ph, const uint8_t *cost) {
+    constexpr uint32_t cnt = 1u << NB;
+    for (uint32_t grp = threadIdx.x; grp < (1u << n) >> NB; grp += blockDim.x) {
+        const uint32_t base = (grp & ((1u << b0) - 1)) | ((grp >> b0) << (b0 + NB)), pb = small_phys(base);
+        float2 a[cnt], l[cnt];
+        float gsum = 0.f;
+#pragma unroll
+        for (uint32_t i = 0; i < cnt; ++i) {
+            const uint32_t at = pb ^ small_phys(i << b0);
+            a[i] = tp[at];
+            if (DUAL) l[i] = tl[at];
+            if (!DUAL && ph) a[i] = cm(a[i], ph[cost[base | (i << b0)]]);
+        }
+#pragma unroll
+        for (uint32_t b = 0; b < (uint32_t)NB; ++b) {
+#pragma unroll
+            for (uint32_t i = 0; i < cnt; ++i) {
+                if (i & (1u << b)) continue;
+                const uint32_t j = i | (1u << b);
+                if (DUAL) gsum += (l[i].x * a[j].y - l[i].y * a[j].x) + (l[j].x * a[i].y - l[j].y * a[i].x);
+                const float2 x = a[i], y = a[j];
+                a[i] = make_float2(c * x.x + s * y.y, c * x.y - s * y.x);
+                a[j] = make_float2(c * y.x + s * x.y, c * y.y - s * x.x);
+                if (DUAL) {
+                    const float2 u = l[i], v = l[j];
+                    l[i] = make_float2(c * u.x + s * v.y, c * u.y - s * v.x);
+                    l[j] = make_float2(c * v.x + s * u.y, c * v.y - s * u.x);
+                }
+            }
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < cnt; ++i) {
+            const uint32_t at = pb ^ small_phys(i << b0);
+            tp[at] = a[i];
+            if (DUAL) tl[at] = l[i];
+        }
+        if (DUAL) g += (double)gsum;
+    }
+    __syncthreads();
+}
+template <bool DUAL>
+__device__ __forceinline__ void small_rounds(float2 *tp, float2 *tl, uint32_t n, uint32_t from, uint32_t to, float c, float s,
+                                             double &g, const float2 *ph, const uint8_t *cost) {
+    for (uint32_t b0 = from; b0 < to; b0 += 4) {
+        switch (min(4u, to - b0)) {
+        case 1: small_round<DUAL, 1>(tp, tl, n, b0, c, s, g, ph, cost); break;
+        case 2: small_round<DUAL, 2>(tp, tl, n, b0, c, s, g, ph, cost); break;
+        case 3: small_round<DUAL, 3>(tp, tl, n, b0, c, s, g, ph, cost); break;
+        default: small_round<DUAL, 4>(tp, tl, n, b0, c, s, g, ph, cost); break;
+        }
+        ph = nullptr;
+    }
+}
+constexpr uint32_t kQSmallTile = 10;  // bits of the first pass
+
+__global__ void __launch_bounds__(kQThreads)
+    k_qaoa_small(const QDesc *__restrict__ desc, const uint64_t *__restrict__ emasks, const double *__restrict__ gammas,
+                 const double *__restrict__ betas, uint32_t p, double *__restrict__ out_cost, double *__restrict__ out_grad) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const QDesc D = desc[blockIdx.x];
+    const uint32_t n = D.n, ne = D.e_count, dim = 1u << n, tid = threadIdx.x;
+    const SmallLayout L = small_layout(n, p, ne);
+    float2 *tp = reinterpret_cast<float2 *>(smem_raw), *tl = reinterpret_cast<float2 *>(smem_raw + L.tl);
+    uint8_t *cost = smem_raw + L.cost;
+    float2 *phase = reinterpret_cast<float2 *>(smem_raw + L.phase);
+    float4 *mixer = reinterpret_cast<float4 *>(smem_raw + L.mixer);
+    uint32_t *em = reinterpret_cast<uint32_t *>(smem_raw + L.emask);
+    double *red = reinterpret_cast<double *>(smem_raw + L.red);
+    const double *gm = gammas + (size_t)D.out * p, *bt = betas + (size_t)D.out * p;
+    for (uint32_t e = tid; e < ne; e += blockDim.x) em[e] = (uint32_t)emasks[D.e_begin + e];
+    // one angle per thread: exp(-i gamma (W - 2c)) of every layer and cut, then the mixers both ways
+    for (uint32_t i = tid; i < p * (ne + 3); i += blockDim.x) {
+        const uint32_t l = i / (ne + 3), c = i % (ne + 3);
+        const double ang = c <= ne ? -gm[l] * ((double)ne - 2.0 * (double)c) : c == ne + 1 ? bt[l] : -bt[l];
+        const float2 f = make_float2((float)cos(ang), (float)sin(ang));
+        if (c <= ne) phase[l * (ne + 1) + c] = f;
+        else reinterpret_cast<float2 *>(mixer)[2 * l + (c - ne - 1)] = f;
+    }
+    __syncthreads();
+    const float amp0 = (float)(1.0 / sqrt((double)dim));
+    for (uint32_t x = tid; x < dim; x += blockDim.x) {
+        tp[small_phys(x)] = make_float2(amp0, 0.f);
+        cost[x] = (uint8_t)cut_value(x, em, ne);
+    }
+    __syncthreads();
+    const uint32_t k = min(n, kQSmallTile);
+    double none = 0.0;
+    for (uint32_t l = 0; l < p; ++l) {
+        const float4 m = mixer[l];
+        small_rounds<false>(tp, tl, n, 0, k, m.x, m.y, none, phase + l * (ne + 1), cost);
+        small_rounds<false>(tp, tl, n, k, n, m.x, m.y, none, nullptr, cost);
+    }
+    // a sum over the block while the others go on: rows of `red` taken in turn
+    auto total = [&](double v, double *row, uint32_t warp, double *out, double factor) {
+        row[tid] = v;
+        __syncthreads();
+        if (tid >> 5 == warp) {
+            double t = 0.0;
+            for (uint32_t j = tid & 31u; j < (uint32_t)kQThreads; j += 32) t += row[j];
+            t = warp_sum(t);
+            if ((tid & 31u) == 0) *out = factor * t;
+        }
+    };
+    double e = 0.0;  // energy, lambda = C psi
+    for (uint32_t x = tid; x < dim; x += blockDim.x) {
+        const float2 a = tp[small_phys(x)];
+        const float cv = (float)cost[x];
+        e += (double)(cv * (a.x * a.x + a.y * a.y));
+        tl[small_phys(x)] = make_float2(cv * a.x, cv * a.y);
+    }
+    total(e, red, 0, out_cost + D.out, 1.0);
+    const float W = (float)ne;
+    double *grad = out_grad + (size_t)D.out * 2 * p;
+    for (uint32_t l = p; l-- > 0;) {
+        const float4 m = mixer[l];
+        const float2 *ph = phase + l * (ne + 1);
+        double gb = 0.0, gg = 0.0;
+        small_rounds<true>(tp, tl, n, k, n, m.z, m.w, gb, nullptr, cost);
+        small_rounds<true>(tp, tl, n, 0, k, m.z, m.w, gb, nullptr, cost);
+        for (uint32_t x = tid; x < dim; x += blockDim.x) {  // the cost layer's gradient, then its phase undone
+            const uint32_t at = small_phys(x);
+            const float2 a = tp[at], v = tl[at];
+            const float gx = W - 2.f * (float)cost[x];
+            gg += (double)(gx * (v.x * a.y - v.y * a.x));
+            const float2 f = ph[cost[x]];
+            tp[at] = cmc(a, f);
+            tl[at] = cmc(v, f);
+        }
+        double *rows = red + (l & 1u) * 2 * kQThreads;  // free again: two barriers lie between
+        total(gg, rows, 1, grad + l, 2.0);
+        total(gb, rows + kQThreads, 2, grad + p + l, 2.0);
+    }
+}
+
 // ---- batched passes for instances of 13..24 qubits ---------------------------
 // All instances of one qubit count n are advanced together, one tile pass per
 // launch over every (instance, tile) pair, so a pass streams at the rate of the
@@ -423,42 +593,52 @@ struct QMix {
 // Phase tables per (instance, layer): forward exp(-i gamma_l (W - 2c)) times
 // the factor its input carries (2^(-n/2) in layer 0, F_{l-1}^n after), at
 // ptab + l * span; the reverse table, times F'_l^n, at ptab + (p + l) * span.
-__global__ void k_qaoa_tables(const QDesc *__restrict__ desc, uint32_t rows, const double *__restrict__ gammas,
-                              const double *__restrict__ betas, uint32_t p, float2 *__restrict__ ptab, QMix *__restrict__ mtab) {
+// The factors (hf, hr) come from a launch of their own, one power per thread:
+// with the powers of every entry computed again the tables took 114 us for 419
+// instances of 4 layers (7 and 15 us now).
+__global__ void k_qaoa_factors(const QDesc *__restrict__ desc, uint32_t rows, const double *__restrict__ betas, uint32_t p,
+                               QMix *__restrict__ mtab, double *__restrict__ hf, double *__restrict__ hr) {
+    const uint64_t per = (uint64_t)rows * p;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < 3 * per; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t which = (uint32_t)(i / per);
+        const uint64_t e = i % per;
+        const QDesc D = desc[e / p];
+        const int n = (int)D.n;
+        const double bt = betas[(size_t)D.out * p + e % p], cb = cos(bt), sb = sin(bt);
+        const bool fc = fabs(cb) >= fabs(sb);
+        const double f = fc ? cb : sb;
+        const double v = pow(which == 0 ? f : which == 1 ? (fc ? cb : -sb) : f * f, which == 2 ? n - kQBTile : n);
+        QMix &M = mtab[e];
+        if (which == 0) {
+            const double k = fc ? sb / cb : cb / sb;
+            M.kf = (float)k;
+            M.kr = (float)-k;
+            M.f2 = (float)(f * f);
+            M.form_c = fc ? 1u : 0u;
+            M.pad = 0;
+            M.fn_f = (float)v;
+            hf[e] = v;
+        } else if (which == 1) {
+            M.fn_r = (float)v;
+            hr[e] = v;
+        } else {
+            M.f2_a0 = (float)v;
+        }
+    }
+}
+__global__ void k_qaoa_tables(const QDesc *__restrict__ desc, uint32_t rows, const double *__restrict__ gammas, uint32_t p,
+                              const double *__restrict__ hf, const double *__restrict__ hr, float2 *__restrict__ ptab) {
     const uint32_t span = kQMaxEdges + 1;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < (uint64_t)rows * p * span;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t r = (uint32_t)(i / ((uint64_t)p * span)), l = (uint32_t)((i / span) % p), c = (uint32_t)(i % span);
         const QDesc D = desc[r];
-        const int n = (int)D.n;
-        auto factor = [&](uint32_t layer, bool inverse) {  // F or F' of a layer's mixer
-            const double bt = betas[(size_t)D.out * p + layer], cb = cos(bt), sb = sin(bt);
-            return fabs(cb) >= fabs(sb) ? cb : (inverse ? -sb : sb);
-        };
-        if (c <= D.e_count) {
-            const double gm = gammas[(size_t)D.out * p + l];
-            const double ang = -gm * ((double)D.e_count - 2.0 * (double)c);
-            const double hin = l == 0 ? 1.0 / sqrt((double)(1ULL << n)) : pow(factor(l - 1, false), n);
-            const double hrev = pow(factor(l, true), n);
-            const double ca = cos(ang), sa = sin(ang);
-            ptab[D.ptab + (uint64_t)l * span + c] = make_float2((float)(hin * ca), (float)(hin * sa));
-            ptab[D.ptab + (uint64_t)(p + l) * span + c] = make_float2((float)(hrev * ca), (float)(hrev * sa));
-        }
-        if (c == 0) {
-            const double bt = betas[(size_t)D.out * p + l], cb = cos(bt), sb = sin(bt);
-            const bool fc = fabs(cb) >= fabs(sb);
-            const double f = fc ? cb : sb, k = fc ? sb / cb : cb / sb;
-            QMix M;
-            M.kf = (float)k;
-            M.kr = (float)-k;
-            M.f2 = (float)(f * f);
-            M.fn_f = (float)pow(f, n);
-            M.fn_r = (float)pow(fc ? cb : -sb, n);
-            M.f2_a0 = (float)pow(f * f, n - kQBTile);
-            M.form_c = fc ? 1u : 0u;
-            M.pad = 0;
-            mtab[(uint64_t)r * p + l] = M;
-        }
+        if (c > D.e_count) continue;
+        const double ang = -gammas[(size_t)D.out * p + l] * ((double)D.e_count - 2.0 * (double)c);
+        const double hin = l == 0 ? 1.0 / sqrt((double)(1ULL << D.n)) : hf[(size_t)r * p + l - 1], hrev = hr[(size_t)r * p + l];
+        const double ca = cos(ang), sa = sin(ang);
+        ptab[D.ptab + (uint64_t)l * span + c] = make_float2((float)(hin * ca), (float)(hin * sa));
+        ptab[D.ptab + (uint64_t)(p + l) * span + c] = make_float2((float)(hrev * ca), (float)(hrev * sa));
     }
 }
 
@@ -832,29 +1012,31 @@ __global__ void __launch_bounds__(kQThreads, 2)
     }
 }
 
-// energy and gradients of the batched instances: per-tile partials in order
+// energy and gradients of the batched instances: one warp per result (one thread
+// each waited on 256 loads in a row: 107 us for 100 instances of 20 qubits, 6 now)
 __global__ void k_qaoa_reduce(const QBArgs a, const QDesc *__restrict__ desc, const double *__restrict__ part,
                               double *__restrict__ out_cost, double *__restrict__ out_grad) {
-    const uint32_t slots = 1 + 2 * a.p;  // energy, dE/dgamma_l, dE/dbeta_l
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < (uint64_t)a.m * slots;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t ci = (uint32_t)(i / slots), sl = (uint32_t)(i % slots);
-        const QDesc D = desc[a.r0 + ci];
+    const uint32_t slots = 1 + 2 * a.p, lane = threadIdx.x & 31u;  // energy, dE/dgamma_l, dE/dbeta_l
+    for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; i < (uint64_t)a.m * slots;
+         i += ((uint64_t)gridDim.x * blockDim.x) >> 5) {
+        const QDesc D = desc[a.r0 + (uint32_t)(i / slots)];
+        const uint32_t sl = (uint32_t)(i % slots);
         const double *P = part + D.part;
-        double v = 0.0;
+        auto row = [&](uint32_t r) {
+            double v = 0.0;
+            for (uint64_t t = lane; t < a.tiles; t += 32) v += P[(uint64_t)r * a.tiles + t];
+            return warp_sum(v);
+        };
         if (sl == 0) {
-            for (uint64_t t = 0; t < a.tiles; ++t) v += P[t];
-            out_cost[D.out] = v;
+            const double v = row(0);
+            if (lane == 0) out_cost[D.out] = v;
         } else if (sl <= a.p) {  // dE/dgamma_l
-            const uint32_t l = sl - 1;
-            for (uint64_t t = 0; t < a.tiles; ++t) v += P[(uint64_t)(1 + 2 * a.p + l) * a.tiles + t];
-            out_grad[(size_t)D.out * 2 * a.p + l] = 2.0 * v;
+            const double v = row(2 * a.p + sl);
+            if (lane == 0) out_grad[(size_t)D.out * 2 * a.p + sl - 1] = 2.0 * v;
         } else {  // dE/dbeta_l: pass A then pass B terms
             const uint32_t l = sl - 1 - a.p;
-            double vb = 0.0;
-            for (uint64_t t = 0; t < a.tiles; ++t) v += P[(uint64_t)(1 + l) * a.tiles + t];
-            for (uint64_t t = 0; t < a.tiles; ++t) vb += P[(uint64_t)(1 + a.p + l) * a.tiles + t];
-            out_grad[(size_t)D.out * 2 * a.p + a.p + l] = 2.0 * (v + vb);
+            const double v = row(1 + l), vb = row(1 + a.p + l);
+            if (lane == 0) out_grad[(size_t)D.out * 2 * a.p + a.p + l] = 2.0 * (v + vb);
         }
     }
 }
@@ -903,15 +1085,17 @@ extern "C" int qf_qaoa_maxcut_batch(qf_ctx *ctx, const qf_qaoa_instance *inst, u
         return I.tile_qubits ? (int)I.tile_qubits : (opts && I.qubits <= 32 ? opts->tile_qubits[I.qubits] : 0);
     };
     auto batched = [&](const qf_qaoa_instance &I) { return I.qubits > (uint32_t)kQBTile && tile_req(I) == 0; };
+    auto rank = [&](const qf_qaoa_instance &I) { return batched(I) ? 0 : tile_req(I) ? 1 : 2; };
     std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) {
-        const bool ba = batched(inst[a]), bb = batched(inst[b]);
-        if (ba != bb) return ba;
+        const int ra = rank(inst[a]), rb = rank(inst[b]);
+        if (ra != rb) return ra < rb;
         return inst[a].qubits > inst[b].qubits;
     });
-    // rows [0, r_small): batched passes per qubit count (13..24 qubits); the
-    // rest: one CTA per instance
+    // rows [0, r_small): batched passes per qubit count (13..24 qubits); then
+    // one CTA per instance: rows of a given tile width, and from r_resident on
+    // those that stay in shared memory
     uint64_t amp_off = 0, cost_off = 0, ptab_off = 0, part_off = 0;
-    uint32_t r_small = 0;
+    uint32_t r_small = 0, r_resident = (uint32_t)n_inst, smem_resident = 0;
     for (uint64_t r = 0; r < n_inst; ++r) {
         const qf_qaoa_instance &I = inst[order[r]];
         QDesc &D = desc[r];
@@ -925,8 +1109,11 @@ extern "C" int qf_qaoa_maxcut_batch(qf_ctx *ctx, const qf_qaoa_instance *inst, u
             ptab_off += 2ULL * p * (kQMaxEdges + 1);  // forward and reverse tables
             D.part = part_off;
             part_off += (uint64_t)(1 + 3 * p) << (D.n - kQBTile);
+        } else if (rank(I) == 2) {
+            r_resident = std::min(r_resident, (uint32_t)r);
+            smem_resident = std::max(smem_resident, small_layout(D.n, p, I.edge_count).total);
         } else {
-            const int kt = tile_req(I) ? tile_req(I) : 10;
+            const int kt = tile_req(I);
             D.k = (uint32_t)std::max(4, std::min(kQMaxTile, kt));
             if (D.n > D.k && D.n - D.k > D.k - 1) D.k = (D.n + 1) / 2 + 1;  // pass B needs n-k+1 <= k
             D.k = std::min<uint32_t>(D.k, (uint32_t)kQMaxTile);
@@ -935,6 +1122,7 @@ extern "C" int qf_qaoa_maxcut_batch(qf_ctx *ctx, const qf_qaoa_instance *inst, u
         D.e_count = I.edge_count;
         D.out = order[r];
         D.pad = 0;
+        if (rank(I) == 2) continue;
         D.psi = amp_off;
         amp_off += 1ULL << D.n;
         D.lam = amp_off;
@@ -950,8 +1138,8 @@ extern "C" int qf_qaoa_maxcut_batch(qf_ctx *ctx, const qf_qaoa_instance *inst, u
     const size_t b_par = al(8 * n_inst * p), b_cost = al(8 * n_inst), b_grad = al(16 * n_inst * p), b_cnt = 256;
     const size_t b_arena = al(8 * amp_off), b_costs = al(cost_off);
     const size_t b_ptab = al(8 * std::max<uint64_t>(1, ptab_off)), b_mtab = al(sizeof(QMix) * std::max<uint64_t>(1, (uint64_t)r_small * p));
-    const size_t b_part = al(8 * std::max<uint64_t>(1, part_off));
-    const size_t total = b_desc + b_mask + 2 * b_par + b_cost + b_grad + b_cnt + b_arena + b_costs + b_ptab + b_mtab + b_part;
+    const size_t b_part = al(8 * std::max<uint64_t>(1, part_off)), b_fac = al(8 * std::max<uint64_t>(1, (uint64_t)r_small * p));
+    const size_t total = 2 * b_fac + b_desc + b_mask + 2 * b_par + b_cost + b_grad + b_cnt + b_arena + b_costs + b_ptab + b_mtab + b_part;
     QF_TRY(ensure_device(&ctx->ws_tree, &ctx->ws_tree_bytes, total));
     unsigned char *w = static_cast<unsigned char *>(ctx->ws_tree);
     QDesc *d_desc = reinterpret_cast<QDesc *>(w);
@@ -967,6 +1155,7 @@ extern "C" int qf_qaoa_maxcut_batch(qf_ctx *ctx, const qf_qaoa_instance *inst, u
     float2 *d_ptab = reinterpret_cast<float2 *>(w2);
     QMix *d_mtab = reinterpret_cast<QMix *>(w2 + b_ptab);
     double *d_part = reinterpret_cast<double *>(w2 + b_ptab + b_mtab);
+    double *d_hf = reinterpret_cast<double *>(w2 + b_ptab + b_mtab + b_part), *d_hr = d_hf + b_fac / 8;
     cudaStream_t st = ctx->stream;
     QF_CUDA(cudaMemcpyAsync(d_desc, desc.data(), sizeof(QDesc) * n_inst, cudaMemcpyHostToDevice, st));
     if (n_edges) QF_CUDA(cudaMemcpyAsync(d_mask, masks.data(), 8 * n_edges, cudaMemcpyHostToDevice, st));
@@ -984,6 +1173,8 @@ extern "C" int qf_qaoa_maxcut_batch(qf_ctx *ctx, const qf_qaoa_instance *inst, u
     const int dev = ctx->device & 63;
     if (!attr[dev]) {
         QF_CUDA(cudaFuncSetAttribute(k_qaoa_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        QF_CUDA(cudaFuncSetAttribute(k_qaoa_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)small_layout(12, kQMaxP, kQMaxEdges).total));
         for (int i = 0; i < 8; ++i) {
             const size_t sm_i = i < 4 ? smem_f : smem_r;
             QF_CUDA(cudaFuncSetAttribute(passes[i], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_i));
@@ -991,7 +1182,7 @@ extern "C" int qf_qaoa_maxcut_batch(qf_ctx *ctx, const qf_qaoa_instance *inst, u
         }
         attr[dev] = true;
     }
-    const uint32_t n_small = (uint32_t)n_inst - r_small;
+    const uint32_t n_small = r_resident - r_small, n_resident = (uint32_t)n_inst - r_resident;
     int per_sm = 0;
     QF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_qaoa_batch, kQThreads, smem));
     const uint32_t grid = (uint32_t)std::min<uint64_t>(std::max(1u, n_small), (uint64_t)std::max(1, per_sm) * ctx->sm_count);
@@ -1003,8 +1194,10 @@ extern "C" int qf_qaoa_maxcut_batch(qf_ctx *ctx, const qf_qaoa_instance *inst, u
     };
     auto enqueue = [&](cudaStream_t s) -> int {
         if (r_small) {
+            k_qaoa_factors<<<(unsigned)std::min<uint64_t>(4096, (3 * (uint64_t)r_small * p + 31) / 32), 32, 0, s>>>(
+                d_desc, r_small, d_bet, p, d_mtab, d_hf, d_hr);
             k_qaoa_tables<<<(unsigned)std::min<uint64_t>(4096, ((uint64_t)r_small * p * (kQMaxEdges + 1) + 255) / 256), 256, 0, s>>>(
-                d_desc, r_small, d_gam, d_bet, p, d_ptab, d_mtab);
+                d_desc, r_small, d_gam, p, d_hf, d_hr, d_ptab);
             QF_CUDA(cudaGetLastError());
         }
         for (uint32_t r0 = 0; r0 < r_small;) {  // one launch sequence per qubit count
@@ -1039,7 +1232,7 @@ extern "C" int qf_qaoa_maxcut_batch(qf_ctx *ctx, const qf_qaoa_instance *inst, u
                 A.chunk = cra;
                 passes[4]<<<gra, kQThreads, smem_r, s>>>(A, d_desc, d_arena, d_costs, d_ptab, d_mtab, d_part);
             }
-            k_qaoa_reduce<<<(unsigned)std::max<uint64_t>(1, ((uint64_t)A.m * (1 + 2 * p) + 127) / 128), 128, 0, s>>>(
+            k_qaoa_reduce<<<(unsigned)std::max<uint64_t>(1, ((uint64_t)A.m * (1 + 2 * p) + 3) / 4), 128, 0, s>>>(
                 A, d_desc, d_part, d_cost, d_grad);
             QF_CUDA(cudaGetLastError());
             r0 = r1;
@@ -1048,6 +1241,10 @@ extern "C" int qf_qaoa_maxcut_batch(qf_ctx *ctx, const qf_qaoa_instance *inst, u
             QF_CUDA(cudaMemsetAsync(d_cnt, 0, sizeof(unsigned), s));
             k_qaoa_batch<<<grid, kQThreads, smem, s>>>(d_desc + r_small, n_small, d_arena, d_costs, d_mask, d_gam, d_bet, p,
                                                        d_cost, d_grad, d_cnt);
+            QF_CUDA(cudaGetLastError());
+        }
+        if (n_resident) {
+            k_qaoa_small<<<n_resident, kQThreads, smem_resident, s>>>(d_desc + r_resident, d_mask, d_gam, d_bet, p, d_cost, d_grad);
             QF_CUDA(cudaGetLastError());
         }
         return QF_OK;
@@ -1066,6 +1263,12 @@ extern "C" int qf_qaoa_maxcut_batch(qf_ctx *ctx, const qf_qaoa_instance *inst, u
         mix(amp_off);
         mix(grid);
         mix(r_small);
+        mix(r_resident);
+        mix(smem_resident);
+        mix((uint64_t)(uintptr_t)d_gam);  // behind the edges: the launches hold every address of the layout
+        mix((uint64_t)(uintptr_t)d_part);
+        mix(cost_off);
+        mix(ptab_off);
         for (uint32_t r = 0; r < r_small; ++r) mix(desc[r].n);
         if (!exec || key != k2) {
             if (exec) cudaGraphExecDestroy(exec);
