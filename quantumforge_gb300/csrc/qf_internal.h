@@ -276,6 +276,7 @@ struct PlanOpts {
     bool merge_1q = true;   // multiply consecutive 1q gates on one qubit
     bool vm = false;        // the plan is for register-tile passes (vm.h)
     bool merge_any = false; // even when the product is a general complex matrix (register-tile passes)
+    bool relabel = false;   // SWAPs may be taken out of the list (absorb_swaps); reorders commuting gates
     bool backward = false;  // adjoint reverse sweep: inverse gates + overlaps
     int max_items = 768;    // bound on ops per pass (shared-memory budget)
     bool search = true;     // choose each pass's resident qubits by look-ahead
