@@ -914,16 +914,20 @@ class Circuit:
         result: (packed outcomes, one u64 per shot with classical bit c at
         bit c; register width; ties)."""
         backend = backend or default_backend()
-        if isinstance(initial_state, StateVector):
-            amps = initial_state.amplitudes()
-        elif isinstance(initial_state, int):
-            amps = np.zeros(1 << initial_state, dtype=np.complex128)
-            amps[0] = 1
+        src = None  # |0...0>, filled on the device
+        if isinstance(initial_state, int) and 1 <= initial_state <= 34:
+            n = int(initial_state)
         else:
-            amps = np.asarray(initial_state, dtype=np.complex128)
-        n = amps.size.bit_length() - 1
+            if isinstance(initial_state, StateVector):
+                amps = initial_state.amplitudes()
+            elif isinstance(initial_state, int):
+                amps = np.zeros(1 << initial_state, dtype=np.complex128)
+                amps[0] = 1
+            else:
+                amps = np.asarray(initial_state, dtype=np.complex128)
+            n = amps.size.bit_length() - 1
+            src = np.ascontiguousarray(amps).view(np.float64)
         ops = self.ops()
-        src = np.ascontiguousarray(amps).view(np.float64)
         out = np.empty(max(int(shots), 1), dtype=np.uint64)
         width = C.c_uint32()
         ties = C.c_uint64()

@@ -6,6 +6,8 @@
 
 #include <complex>
 #include <cstdint>
+#include <map>
+#include <mutex>
 #include <set>
 #include <string>
 #include <vector>
@@ -28,6 +30,9 @@ struct qf_ctx {
     qf_sv *scratch_sv = nullptr;  // cached state for whole-circuit calls
     qf_sv *scratch_sv2 = nullptr; // cached second state (adjoint costate)
     std::set<qf_sv *> states;     // live states; orphaned (memory freed) when the context is destroyed
+    std::mutex pool_mu;              // guards the two below
+    std::multimap<size_t, void *> free_blocks;  // memory of destroyed states, by bytes (bounded; kStatePoolBytes)
+    size_t free_bytes = 0;
     std::vector<qf_sv *> ckpt_pool;  // adjoint checkpoint states kept for the next gradient (bounded bytes)
 };
 constexpr size_t kSmallBytes = 64 * 1024;
@@ -38,6 +43,7 @@ struct qf_sv {
     int dtype = QF_C64;
     uint64_t dim = 0;
     void *d = nullptr;  // 2^n complex amplitudes, interleaved
+    bool exposed = false;  // its address was given out: the memory goes back to the device with the state
     size_t bytes() const { return dim * (dtype == QF_C64 ? 8u : 16u); }
 };
 

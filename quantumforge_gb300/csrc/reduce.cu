@@ -52,12 +52,19 @@ static int partials_buffer(qf_ctx *ctx, size_t doubles, double **out) {
 template <typename C> __device__ __forceinline__ typename Real<C>::T nsq(C a) { return a.x * a.x + a.y * a.y; }
 
 // ---- state fill / conversion ---------------------------------------------
-template <typename C> __global__ void k_set_first_one(C *a) { a[0] = mk((typename Real<C>::T)1, (typename Real<C>::T)0); }
+// |0...0> in one launch (a memset and a kernel for the first amplitude cost a
+// small state two launches and the gap between them)
+__global__ void k_zero_state(uint4 *a, uint64_t words, uint32_t one_hi, uint32_t one_lo) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < words; i += (uint64_t)gridDim.x * blockDim.x)
+        a[i] = i == 0 ? make_uint4(one_lo, one_hi, 0, 0) : make_uint4(0, 0, 0, 0);
+}
 
 int fill_zero_state(qf_sv *sv) {
-    QF_CUDA(cudaMemsetAsync(sv->d, 0, sv->bytes(), sv->ctx->stream));
-    if (sv->dtype == QF_C64) k_set_first_one<float2><<<1, 1, 0, sv->ctx->stream>>>(static_cast<float2 *>(sv->d));
-    else k_set_first_one<double2><<<1, 1, 0, sv->ctx->stream>>>(static_cast<double2 *>(sv->d));
+    const uint64_t words = sv->bytes() / 16;  // at least two amplitudes
+    const bool f = sv->dtype == QF_C64;       // 1.0f, or 1.0 (low word zero)
+    const uint64_t blocks = std::min<uint64_t>((words + 255) / 256, (uint64_t)sv->ctx->sm_count * 8);
+    k_zero_state<<<(unsigned)blocks, 256, 0, sv->ctx->stream>>>(static_cast<uint4 *>(sv->d), words, f ? 0u : 0x3FF00000u,
+                                                                 f ? 0x3F800000u : 0u);
     QF_CUDA(cudaGetLastError());
     return QF_OK;
 }
