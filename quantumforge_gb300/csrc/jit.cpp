@@ -718,6 +718,11 @@ struct PassGen {
             s << "float2* S = SB;\nfloat2* SL = SB + " << tile_of(K) << "u;\n";
         }
         s << "const unsigned long long tb = " << dep_t << ";\n";
+        if (dual && p.a.n_slots) {
+            s << "float op0 = 0.f";
+            for (int k = 1; k < kOvlBatch; ++k) s << ", op" << k << " = 0.f";
+            s << ";\n";
+        }
         s << "float2 tph = make_float2(1.f, 0.f);\n";  // deferred per-thread phase (psi and lambda alike)
         phase_pending = false;
         for (int a = 0; a < n_arrays(); ++a)
@@ -792,8 +797,7 @@ struct PassGen {
 
     // Im<lambda|P_q psi> over the thread's amplitudes (the adjoint term of
     // src/lib.rs:3648-3664, summed as the shared-memory kernel does), reduced
-    // over the warp in f32 and added to the slot's f64 accumulator (held by
-    // lane slot % 32).
+    // over the warp in f32 and added to a float-pair accumulator (flush_overlaps).
     // Z-axis overlaps of a backward pass are held back until nothing else can
     // run, then evaluated together: Im<lambda|Z_q psi> commutes with every gate
     // still pending before it (none of them acts off-diagonal on q), and all of
@@ -849,10 +853,37 @@ struct PassGen {
             const int sl = g.slot(std::norm(g.pscale), 0.0, 0.0, 0.0);
             s << "ov *= " << Mref(sl, 0) << ".x;\n";
         }
-        for (int o = 16; o >= 1; o >>= 1) s << "ov += __shfl_xor_sync(0xffffffffu, ov, " << o << ");\n";
-        const std::string ah = "acc" + std::to_string(ls >> 5) + "h", al = "acc" + std::to_string(ls >> 5) + "l";
-        s << "if (lane == " << (ls & 31) << "u) {const float sm = " << ah << " + ov, bb = sm - " << ah << "; " << al << " += ("
-          << ah << " - (sm - bb)) + (ov - bb); " << ah << " = sm;}\n";
+        s << "op" << waiting << " = ov;\n";
+        slot_of_order.push_back(ls);
+        if (++waiting == kOvlBatch) flush_overlaps();
+    }
+    // The waiting overlaps' warp sums, kOvlBatch at a time: at each butterfly step
+    // that still has several values a lane keeps half of them and hands the other
+    // half over, so every value is added up in the same tree as alone, with 9
+    // shuffles for eight instead of 40, and one float-pair addition. Lane l then
+    // holds value l / (32 / kOvlBatch); batches take the lanes of one residue each.
+    // (One by one: 24-qubit gradient 3.80 ms, 28 qubits 50.5; eight 3.51 and 49.3;
+    // four 3.55 and 49.1; sixteen 3.54 and 50.6, with spills.)
+    static constexpr int kOvlBatch = 8;
+    int waiting = 0;
+    std::vector<int> slot_of_order;  // overlaps in order of emission
+    void flush_overlaps() {
+        if (!waiting) return;
+        auto &s = g.s;
+        s << "{";
+        for (int k = waiting; k < kOvlBatch; ++k) s << "op" << k << " = 0.f; ";
+        int o = 16;
+        for (int m = kOvlBatch / 2; m >= 1; m >>= 1, o >>= 1)
+            for (int k = 0; k < m; ++k)
+                s << "{const bool h = (lane & " << o << "u) != 0; const float keep = h ? op" << k + m << " : op" << k << ", give = h ? op" << k
+                  << " : op" << k + m << "; op" << k << " = keep + __shfl_xor_sync(0xffffffffu, give, " << o << ");}\n";
+        for (; o >= 1; o >>= 1) s << "op0 += __shfl_xor_sync(0xffffffffu, op0, " << o << ");\n";
+        constexpr int share = 32 / kOvlBatch;
+        const int batch = ((int)slot_of_order.size() - 1) / kOvlBatch;
+        const std::string ah = "acc" + std::to_string(batch / share) + "h", al = "acc" + std::to_string(batch / share) + "l";
+        s << "if ((lane & " << share - 1 << "u) == " << batch % share << "u) {const float sm = " << ah << " + op0, bb = sm - " << ah << "; "
+          << al << " += (" << ah << " - (sm - bb)) + (op0 - bb); " << ah << " = sm;}}\n";
+        waiting = 0;
     }
 
     void emit_overlap(const BGate &x) {
@@ -1069,6 +1100,7 @@ struct PassGen {
 
     void finish(bool last_pass, const std::string &dep_t2) {
         auto &s = g.s;
+        flush_overlaps();
         flush_phase();
         if (last_pass && g.any_diag) {  // the plan's global phase, once, at the very end (with this pass's factors)
             const int sl = g.slot(g.gphase * g.pscale, 0.0, 0.0, 0.0);
@@ -1129,9 +1161,15 @@ struct PassGen {
         if (dual) {  // per-CTA slot sums, warps in order
             s << "asm volatile(\"cp.async.wait_group 0;\\n\" ::: \"memory\");\n__syncthreads();\n";
             s << "double* RD = reinterpret_cast<double*>(SB);\n";
-            for (int a = 0; a < n_acc(); ++a)
-                s << "if (lane + " << 32 * a << "u < " << p.a.n_slots << "u) RD[(lane + " << 32 * a << "u) * 8u + warp] = (double)acc"
-                  << a << "h + (double)acc" << a << "l;\n";
+            constexpr int share = 32 / kOvlBatch;
+            for (int a = 0; a < n_acc(); ++a) {  // lane -> slot of the overlap it holds
+                s << "{const unsigned short so[32] = {";
+                for (int l = 0; l < 32; ++l) {
+                    const size_t at = (size_t)(a * share + l % share) * kOvlBatch + l / share;
+                    s << (l ? "," : "") << (at < slot_of_order.size() ? slot_of_order[at] : 0xFFFF);
+                }
+                s << "}; const unsigned k = so[lane]; if (k != 65535u) RD[k * 8u + warp] = (double)acc" << a << "h + (double)acc" << a << "l;}\n";
+            }
             s << "__syncthreads();\n";
             s << "for (unsigned k = tid; k < " << p.a.n_slots << "u; k += " << threads_of(K) << "u) {double v = 0.0;"
               << " for (unsigned w = 0; w < 8u; ++w) v += RD[k * 8u + w];"
