@@ -582,6 +582,7 @@ struct PassGen {
     static const char *reg_pfx(int a) { return a ? "l" : "r"; }
     static const char *smem_of(int a) { return a ? "SL" : "S"; }
     static const char *glob_of(int a) { return a ? "B" : "A"; }
+    const char *store_of(int a) const { return dual ? glob_of(a) : "O"; }
     // read all registers from shared memory in the current layout
     void emit_read() {
         std::copy(L, L + kPosMax, read_L);
@@ -671,7 +672,7 @@ struct PassGen {
         if (!dual)
             s << "extern \"C\" __global__ void __launch_bounds__(" << threads_of(K) << ", "
               << (K == 12 ? (p.max_block >= 2 ? 2 : 3) : 1) << ") p" << index
-              << "(float2* __restrict__ A, unsigned long long nt) {\n";
+              << "(const float2* A, float2* O, unsigned long long nt) {\n";  // O: A, or another state
         else
             s << "extern \"C\" __global__ void __launch_bounds__(" << threads_of(K) << ", 2) b" << index
               << "(float2* __restrict__ A, float2* __restrict__ B, unsigned long long nt, double* __restrict__ partials, "
@@ -1139,7 +1140,7 @@ struct PassGen {
                     uint64_t off = 0;
                     for (int r = 0; r < 4; ++r)
                         if ((i >> r) & 1) off |= 1ULL << L[5 + r];
-                    s << glob_of(a) << "[(tb | lane | sw) | " << hex64(off) << "] = " << g.R(i) << ";\n";
+                    s << store_of(a) << "[(tb | lane | sw) | " << hex64(off) << "] = " << g.R(i) << ";\n";
                 }
             }
             g.pfx = "r";
@@ -1148,7 +1149,7 @@ struct PassGen {
             s << "__syncthreads();\n";
             for (int a = 0; a < n_arrays(); ++a)
                 for (int k = 0; k < kChunks; ++k)
-                    s << "*reinterpret_cast<float4*>(" << glob_of(a) << " + (tb | toff | " << hex64(chunk_k_bits(k))
+                    s << "*reinterpret_cast<float4*>(" << store_of(a) << " + (tb | toff | " << hex64(chunk_k_bits(k))
                       << ")) = *reinterpret_cast<const float4*>(" << smem_of(a) << " + (pt2 ^ " << physj(chunk_j(k)) << "u));\n";
             s << "__syncthreads();\n";
             if (dual) {
@@ -1546,13 +1547,17 @@ int grid_of(qf_ctx *ctx, cudaKernel_t k, int K, uint64_t n_tiles, uint64_t *grid
 }  // namespace
 
 // Generate, compile (or fetch) and launch the plan's passes.
-int run_plan_jit(qf_sv *sv, const Plan &plan, int) {
+int run_plan_jit(qf_sv *sv, const Plan &plan, int, const qf_sv *src) {
     const int wb = (int)plan.passes[0].a.k - 9;
     // interpreted when the plan does not fit the compiled layout
-    if (!jit_plan_fits(plan)) return plan.block_qubits ? run_plan_blocks(sv, plan) : run_plan_rs(sv, plan, wb);
+    auto interpreted = [&]() -> int {
+        QF_TRY(copy_from(sv, src));
+        return plan.block_qubits ? run_plan_blocks(sv, plan) : run_plan_rs(sv, plan, wb);
+    };
+    if (!jit_plan_fits(plan)) return interpreted();
     qf_ctx *ctx = sv->ctx;
     std::vector<ModulePlan> mods;
-    if (!gen_modules(plan, mods)) return plan.block_qubits ? run_plan_blocks(sv, plan) : run_plan_rs(sv, plan, wb);
+    if (!gen_modules(plan, mods)) return interpreted();
     std::vector<std::shared_ptr<JitModule>> handles;
     QF_TRY(fetch_modules(ctx, mods, handles));
     for (size_t m = 0; m < mods.size(); ++m) {
@@ -1564,8 +1569,10 @@ int run_plan_jit(qf_sv *sv, const Plan &plan, int) {
             const int K = pass_k(p);
             QF_TRY(grid_of(ctx, jm.kernels[k], K, p.a.n_tiles, &grid));
             float2 *amps = static_cast<float2 *>(sv->d);
+            const float2 *from = src ? static_cast<const float2 *>(src->d) : amps;
+            src = nullptr;  // the first pass only
             unsigned long long nt = p.a.n_tiles;
-            void *args[] = {&amps, &nt};
+            void *args[] = {&from, &amps, &nt};
             QF_CUDA(cudaLaunchKernel((const void *)jm.kernels[k], dim3((unsigned)grid), dim3(threads_of(K)), args, dyn_smem_of(K),
                                      ctx->stream));
         }

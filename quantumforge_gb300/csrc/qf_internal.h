@@ -312,8 +312,11 @@ void sweep_tiling(uint32_t n, int dtype, const qf_exec_opts *opts, bool dual, bo
 // Unfused single-gate sweeps.
 int launch_gate1(qf_sv *sv, const BGate &g);
 int launch_gate2(qf_sv *sv, const BGate &g);
-// Run every pass of a plan on the engine it was made for (sweep_tiling).
-int run_plan(qf_sv *sv, const Plan &plan, int flags = 0);
+// Run every pass of a plan on the engine it was made for (sweep_tiling). With
+// `src`, another state of the same shape, sv becomes the plan's result on src:
+// the first compiled pass reads src itself, the other engines a copy.
+int run_plan(qf_sv *sv, const Plan &plan, int flags = 0, const qf_sv *src = nullptr);
+int copy_from(qf_sv *sv, const qf_sv *src);  // nothing without src
 int run_plan_smem(qf_sv *sv, const Plan &plan);
 // Plans with dense blocks: the shared-memory block interpreter (any width,
 // complex64 and complex128) and, for complex64 blocks of 5 qubits, the
@@ -326,7 +329,7 @@ int run_plan_blocks_mma(qf_sv *sv, const Plan &plan);
 constexpr uint32_t kJitMinQubits = 24;
 bool jit_available();
 int run_plan_rs(qf_sv *sv, const Plan &plan, int wb);
-int run_plan_jit(qf_sv *sv, const Plan &plan, int wb);
+int run_plan_jit(qf_sv *sv, const Plan &plan, int wb, const qf_sv *src = nullptr);
 // Generate the plan's pass kernels and compile them with NVRTC without
 // loading them (no GPU needed); for tests of the code generator. `dual`
 // generates the backward (psi, lambda) kernels of an adjoint plan.

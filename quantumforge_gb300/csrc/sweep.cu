@@ -796,28 +796,29 @@ int run_plan_smem(qf_sv *sv, const Plan &plan) {
     return launch_passes<double2, false>(sv, nullptr, plan, nullptr);
 }
 
-int run_plan(qf_sv *sv, const Plan &plan, int flags) {
-    if (plan.passes.empty()) return QF_OK;
+int copy_from(qf_sv *sv, const qf_sv *src) {
+    if (src) QF_CUDA(cudaMemcpyAsync(sv->d, src->d, sv->bytes(), cudaMemcpyDeviceToDevice, sv->ctx->stream));
+    return QF_OK;
+}
+
+int run_plan(qf_sv *sv, const Plan &plan, int flags, const qf_sv *src) {
+    if (plan.passes.empty()) return copy_from(sv, src);
+    const uint32_t k = plan.passes[0].a.k;
+    const bool tiles64 = sv->dtype == QF_C64 && !(flags & QF_EXEC_FLAG_SMEM_TILES);
+    // compiled passes for large states (the compile is amortised over many
+    // sweeps of the state)
+    const bool jit = tiles64 && sv->n >= 12 && !(flags & QF_EXEC_FLAG_NO_JIT) &&
+                     ((flags & QF_EXEC_FLAG_JIT) || sv->n >= kJitMinQubits) && jit_available();
     if (plan.block_qubits) {  // dense k-qubit blocks
-        if (sv->dtype == QF_C64 && !(flags & QF_EXEC_FLAG_SMEM_TILES)) {
-            if (plan.block_qubits == 5 && !(flags & QF_EXEC_FLAG_BLOCKS_SIMT) && mma_blocks_fit(plan))
-                return run_plan_blocks_mma(sv, plan);
-            if (plan.block_qubits <= 4 && sv->n >= 12 && plan.passes[0].a.k == 12 && !(flags & QF_EXEC_FLAG_NO_JIT) &&
-                ((flags & QF_EXEC_FLAG_JIT) || sv->n >= kJitMinQubits) && jit_available())
-                return run_plan_jit(sv, plan, 3);
-        }
-        return run_plan_blocks(sv, plan);
+        const bool mma = tiles64 && plan.block_qubits == 5 && !(flags & QF_EXEC_FLAG_BLOCKS_SIMT) && mma_blocks_fit(plan);
+        if (!mma && jit && plan.block_qubits <= 4 && k == 12) return run_plan_jit(sv, plan, 3, src);
+        QF_TRY(copy_from(sv, src));
+        return mma ? run_plan_blocks_mma(sv, plan) : run_plan_blocks(sv, plan);
     }
+    if (!plan.vm && jit && (k == 12 || k == 13)) return run_plan_jit(sv, plan, 3, src);
+    QF_TRY(copy_from(sv, src));
     if (plan.vm) return run_plan_vm(sv, plan);
-    if (sv->dtype == QF_C64 && !(flags & QF_EXEC_FLAG_SMEM_TILES) && sv->n >= 12) {
-        const uint32_t k = plan.passes[0].a.k;
-        // compiled passes for large states (the compile is amortised over many
-        // sweeps of the state)
-        const bool jit = (k == 12 || k == 13) && !(flags & QF_EXEC_FLAG_NO_JIT) &&
-                         ((flags & QF_EXEC_FLAG_JIT) || sv->n >= kJitMinQubits) && jit_available();
-        if (jit) return run_plan_jit(sv, plan, 3);
-        if (k == 12 || k == 13) return run_plan_rs(sv, plan, (int)k - 9);
-    }
+    if (tiles64 && sv->n >= 12 && (k == 12 || k == 13)) return run_plan_rs(sv, plan, (int)k - 9);
     return run_plan_smem(sv, plan);
 }
 
