@@ -366,7 +366,9 @@ int adjoint_device(qf_ctx *ctx, uint32_t n, const std::vector<BGate> &gates, con
     QF_TRY(pauli_apply(psi, lam, terms, n_terms, nullptr, d_sums + total_slots));
     if (total_slots) QF_CUDA(cudaMemsetAsync(d_sums, 0, bytes, ctx->stream));
     for (size_t s = n_seg; s-- > 0;) {
-        QF_TRY(run_plan_dual(psi, lam, bplans[s], bplans[s].n_slots ? d_sums + slot_off[s] : nullptr, o->exec.flags));
+        // behind a segment's last pass psi comes from a checkpoint, behind the first segment nothing is needed
+        const unsigned keep = s == 0 ? 0u : !ckpt.empty() ? 2u : 3u;
+        QF_TRY(run_plan_dual(psi, lam, bplans[s], bplans[s].n_slots ? d_sums + slot_off[s] : nullptr, o->exec.flags, keep));
         if (s > 0 && !ckpt.empty()) std::swap(psi->d, ckpt[s - 1]->d);  // psi at the segment's start
     }
     std::vector<double> sums(total_slots + 2);

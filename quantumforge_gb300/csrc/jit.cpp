@@ -582,6 +582,7 @@ struct PassGen {
     static const char *reg_pfx(int a) { return a ? "l" : "r"; }
     static const char *smem_of(int a) { return a ? "SL" : "S"; }
     static const char *glob_of(int a) { return a ? "B" : "A"; }
+    std::string store_if(int a) const { return dual ? "if (keep & " + std::to_string(1 << a) + "u) " : ""; }
     const char *store_of(int a) const { return dual ? glob_of(a) : "O"; }
     // read all registers from shared memory in the current layout
     void emit_read() {
@@ -676,7 +677,7 @@ struct PassGen {
         else
             s << "extern \"C\" __global__ void __launch_bounds__(" << threads_of(K) << ", 2) b" << index
               << "(float2* __restrict__ A, float2* __restrict__ B, unsigned long long nt, double* __restrict__ partials, "
-                 "unsigned stride) {\n";
+                 "unsigned stride, unsigned keep) {\n";  // keep: bit 0 store psi, bit 1 store lambda
         s << "extern __shared__ __align__(16) float2 SB[];\n";
         s << "const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, tid = threadIdx.x;\n";
         s << "const unsigned sbase = (unsigned)__cvta_generic_to_shared(SB);\n";
@@ -1136,12 +1137,14 @@ struct PassGen {
             s << ";\n";
             for (int a = 0; a < n_arrays(); ++a) {
                 g.pfx = reg_pfx(a);
+                s << store_if(a) << "{\n";
                 for (int i = 0; i < kR; ++i) {
                     uint64_t off = 0;
                     for (int r = 0; r < 4; ++r)
                         if ((i >> r) & 1) off |= 1ULL << L[5 + r];
                     s << store_of(a) << "[(tb | lane | sw) | " << hex64(off) << "] = " << g.R(i) << ";\n";
                 }
+                s << "}\n";
             }
             g.pfx = "r";
         } else {  // through shared memory, 16-byte coalesced stores
@@ -1149,7 +1152,7 @@ struct PassGen {
             s << "__syncthreads();\n";
             for (int a = 0; a < n_arrays(); ++a)
                 for (int k = 0; k < kChunks; ++k)
-                    s << "*reinterpret_cast<float4*>(" << store_of(a) << " + (tb | toff | " << hex64(chunk_k_bits(k))
+                    s << store_if(a) << "*reinterpret_cast<float4*>(" << store_of(a) << " + (tb | toff | " << hex64(chunk_k_bits(k))
                       << ")) = *reinterpret_cast<const float4*>(" << smem_of(a) << " + (pt2 ^ " << physj(chunk_j(k)) << "u));\n";
             s << "__syncthreads();\n";
             if (dual) {
@@ -1583,7 +1586,7 @@ int run_plan_jit(qf_sv *sv, const Plan &plan, int, const qf_sv *src) {
 // Backward adjoint passes: psi and lambda in registers, the overlap slots
 // reduced per CTA into partials[slot * stride + block] and then summed in
 // block order into d_slot_sums.
-int run_plan_jit_dual(qf_sv *psi, qf_sv *lam, const Plan &plan, double *d_slot_sums) {
+int run_plan_jit_dual(qf_sv *psi, qf_sv *lam, const Plan &plan, double *d_slot_sums, unsigned keep) {
     if (!jit_plan_fits(plan, true)) return run_plan_dual_smem(psi, lam, plan, d_slot_sums);
     qf_ctx *ctx = psi->ctx;
     std::vector<ModulePlan> mods;
@@ -1610,7 +1613,8 @@ int run_plan_jit_dual(qf_sv *psi, qf_sv *lam, const Plan &plan, double *d_slot_s
             unsigned long long nt = p.a.n_tiles;
             double *parts = d_partials;
             unsigned str = stride;
-            void *args[] = {&a, &b, &nt, &parts, &str};
+            unsigned stored = m + 1 == mods.size() && k + 1 == mods[m].pass_index.size() ? keep : 3u;
+            void *args[] = {&a, &b, &nt, &parts, &str, &stored};
             QF_CUDA(cudaLaunchKernel((const void *)jm.kernels[k], dim3((unsigned)grid), dim3(threads_of(K)), args, dyn_smem_of(K),
                                      ctx->stream));
         }

@@ -339,7 +339,9 @@ int jit_check_compile(const Plan &plan, int wb, std::string *source, std::string
 // Complex64 states use compiled dual passes (by default from kJitMinQubits
 // qubits, or with QF_EXEC_FLAG_JIT; QF_EXEC_FLAG_SMEM_TILES forces the
 // shared-memory kernel).
-int run_plan_dual(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_slot_sums, int flags = 0);
+// `keep`: what of psi (1) and lambda (2) the caller still needs; compiled passes
+// leave the rest unwritten at the end of the plan.
+int run_plan_dual(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_slot_sums, int flags = 0, unsigned keep = 3);
 int run_plan_dual_smem(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_slot_sums);
 // The same passes in groups of ops that share one assignment of amplitudes to
 // threads (complex64; dualpass.cu); plans it does not cover run on the
@@ -347,7 +349,7 @@ int run_plan_dual_smem(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_sl
 int run_plan_dual_groups(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_slot_sums);
 // Compiled backward passes; falls back to run_plan_dual_smem for plans the
 // compiled layout does not cover.
-int run_plan_jit_dual(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_slot_sums);
+int run_plan_jit_dual(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_slot_sums, unsigned keep = 3);
 // slot_sums[s] += sum over b < stride of partials[s * stride + b] (block order)
 int reduce_slots(qf_ctx *ctx, const double *partials, uint32_t stride, uint32_t n_slots, double *d_slot_sums);
 

@@ -827,14 +827,14 @@ int run_plan_dual_smem(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_sl
     return launch_passes<double2, true>(psi, lambda, plan, d_slot_sums);
 }
 
-int run_plan_dual(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_slot_sums, int flags) {
+int run_plan_dual(qf_sv *psi, qf_sv *lambda, const Plan &plan, double *d_slot_sums, int flags, unsigned keep) {
     if (plan.passes.empty()) return QF_OK;
     if (psi->dtype != lambda->dtype || psi->n != lambda->n)
         return fail(QF_ERR_INCOMPATIBLE_DEVICE_STATE, "device states must have equal dimensions and dtype");
     if (plan.vm) return run_plan_vm_dual(psi, lambda, plan, d_slot_sums);
     if (psi->dtype == QF_C64 && !(flags & QF_EXEC_FLAG_SMEM_TILES) && !(flags & QF_EXEC_FLAG_NO_JIT) &&
         ((flags & QF_EXEC_FLAG_JIT) || psi->n >= kJitMinQubits) && jit_available())
-        return run_plan_jit_dual(psi, lambda, plan, d_slot_sums);
+        return run_plan_jit_dual(psi, lambda, plan, d_slot_sums, keep);
     if (psi->dtype == QF_C64 && !(flags & QF_EXEC_FLAG_SMEM_TILES)) return run_plan_dual_groups(psi, lambda, plan, d_slot_sums);
     return run_plan_dual_smem(psi, lambda, plan, d_slot_sums);
 }
