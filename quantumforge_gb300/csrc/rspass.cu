@@ -69,6 +69,9 @@ __device__ __forceinline__ BitSrc bit_src(uint8_t d, uint32_t lane, uint32_t war
 }
 __device__ __forceinline__ int bit_of(const BitSrc &s, int i) { return s.reg >= 0 ? (i >> s.reg) & 1 : s.konst; }
 
+// amplitudes whose register bit r is set, one bit each
+__device__ __forceinline__ uint32_t ones_of(int r) { return r == 0 ? 0xAAAAu : r == 1 ? 0xCCCCu : r == 2 ? 0xF0F0u : 0xFF00u; }
+__device__ __forceinline__ uint32_t pattern(const BitSrc &s) { return s.reg >= 0 ? ones_of(s.reg) : s.konst ? 0xFFFFu : 0u; }
 template <int B>
 __device__ __forceinline__ void reg_cnot(float2 (&r)[kRsRegs], const BitSrc &c) {
 #pragma unroll
@@ -82,7 +85,6 @@ __device__ __forceinline__ void reg_cnot(float2 (&r)[kRsRegs], const BitSrc &c) 
             }
         }
 }
-
 template <int B>
 __device__ __forceinline__ void reg_swap_lane(float2 (&r)[kRsRegs], uint32_t lane, int a) {
     const int la = (lane >> a) & 1;
@@ -102,7 +104,11 @@ __device__ __forceinline__ void reg_swap_lane(float2 (&r)[kRsRegs], uint32_t lan
 
 __device__ __forceinline__ uint32_t layout_offset(uint32_t packed, int pos) { return (packed >> (3 * pos)) & 7u; }
 
-template <int WB>
+// CZ: the pass has CZ gates. Their signs gather in a bit per amplitude and are
+// applied before the next op that mixes or moves amplitudes (20 qubits, 4 layers
+// with a CZ ring: 157 us of passes, now 127; passes without CZ ran 7 % slower with
+// the test for waiting signs, so they have a kernel without it).
+template <int WB, bool CZ>
 __global__ void __launch_bounds__(32 << WB, (WB == 3 ? 2 : 1))
     k_rs_pass(float2 *__restrict__ amps, const RsPassArgs pa, const RsOp *__restrict__ g_ops,
               const double *__restrict__ g_mats) {
@@ -156,8 +162,21 @@ __global__ void __launch_bounds__(32 << WB, (WB == 3 ? 2 : 1))
                 r[i] = amps[base | off];
             }
         }
+        uint32_t signs = 0;
+        bool pending = false;  // uniform over the CTA
+        auto apply_signs = [&] {
+            if (!CZ || !pending) return;
+            pending = false;
+#pragma unroll
+            for (int i = 0; i < kRsRegs; ++i) {
+                const uint32_t m = (signs << (31 - i)) & 0x80000000u;
+                r[i] = make_float2(__uint_as_float(__float_as_uint(r[i].x) ^ m), __uint_as_float(__float_as_uint(r[i].y) ^ m));
+            }
+            signs = 0;
+        };
         for (uint32_t o = 0; o < pa.n_ops; ++o) {
             const RsOp op = ops[o];
+            if (CZ && op.kind != RS_DIAG && op.kind != RS_CZ) apply_signs();
             switch (op.kind) {
             case RS_MREG: {
                 const RsMat M = mats[op.mat];
@@ -223,10 +242,10 @@ __global__ void __launch_bounds__(32 << WB, (WB == 3 ? 2 : 1))
                 break;
             }
             case RS_CZ: {
+                if (!CZ) break;
                 const BitSrc a = bit_src(op.p0, lane, warp, tb), b = bit_src(op.p1, lane, warp, tb);
-#pragma unroll
-                for (int i = 0; i < kRsRegs; ++i)
-                    if (bit_of(a, i) & bit_of(b, i)) r[i] = cneg(r[i]);
+                signs ^= pattern(a) & pattern(b);
+                pending = true;
                 break;
             }
             case RS_SWAP_LR: {
@@ -280,6 +299,7 @@ __global__ void __launch_bounds__(32 << WB, (WB == 3 ? 2 : 1))
             }
             }
         }
+        apply_signs();
         if (cross_warp) __syncthreads();
         {
             const uint64_t base = tb | lane | sw;
@@ -300,7 +320,11 @@ static size_t rs_smem(int wb, uint32_t n_ops, uint32_t n_mats) {
 template <int WB> static int rs_launch_all(qf_sv *sv, const RsPlan &rp, const Plan &plan) {
     qf_ctx *ctx = sv->ctx;
     static size_t dyn[64] = {0};
-    if (!dyn[ctx->device & 63]) QF_TRY(allow_max_dynamic_smem(k_rs_pass<WB>, ctx, &dyn[ctx->device & 63]));
+    if (!dyn[ctx->device & 63]) {
+        size_t both = 0;
+        QF_TRY(allow_max_dynamic_smem(k_rs_pass<WB, false>, ctx, &both));
+        QF_TRY(allow_max_dynamic_smem(k_rs_pass<WB, true>, ctx, &dyn[ctx->device & 63]));
+    }
     const size_t ops_b = (rp.ops.size() * sizeof(RsOp) + 15) / 16 * 16;
     const size_t mats_b = rp.mats.size() * sizeof(double);
     QF_TRY(ensure_device(&ctx->ws_plan, &ctx->ws_plan_bytes, ops_b + mats_b + 16));
@@ -316,14 +340,19 @@ template <int WB> static int rs_launch_all(qf_sv *sv, const RsPlan &rp, const Pl
         if (!p.fallback) max_smem = std::max(max_smem, rs_smem(WB, p.a.n_ops, p.a.n_mats));
     if (max_smem > dyn[ctx->device & 63])
         return fail(QF_ERR_UNSUPPORTED_OPERATION, "register-tiled pass needs %zu bytes of shared memory", max_smem);
-    int per_sm = 0;
-    QF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_rs_pass<WB>, 32 << WB, max_smem));
-    per_sm = std::max(per_sm, 1);
-    const uint64_t grid = (uint64_t)per_sm * ctx->sm_count;
+    uint64_t grid[2];
+    for (int cz = 0; cz < 2; ++cz) {
+        int per_sm = 0;
+        QF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cz ? k_rs_pass<WB, true> : k_rs_pass<WB, false>, 32 << WB,
+                                                              max_smem));
+        grid[cz] = (uint64_t)std::max(per_sm, 1) * ctx->sm_count;
+    }
     for (size_t i = 0; i < rp.passes.size(); ++i) {
         const RsPass &p = rp.passes[i];
-        const uint32_t g = (uint32_t)std::min<uint64_t>(grid, p.a.n_tiles);
-        k_rs_pass<WB><<<g, 32 << WB, rs_smem(WB, p.a.n_ops, p.a.n_mats), ctx->stream>>>(
+        bool cz = false;
+        for (uint32_t o = 0; o < p.a.n_ops; ++o) cz |= rp.ops[p.op_begin + o].kind == RS_CZ;
+        const uint32_t g = (uint32_t)std::min<uint64_t>(grid[cz], p.a.n_tiles);
+        (cz ? k_rs_pass<WB, true> : k_rs_pass<WB, false>)<<<g, 32 << WB, rs_smem(WB, p.a.n_ops, p.a.n_mats), ctx->stream>>>(
             static_cast<float2 *>(sv->d), p.a, d_ops + p.op_begin, d_mats + 8 * (size_t)p.mat_begin);
         QF_CUDA(cudaGetLastError());
     }
