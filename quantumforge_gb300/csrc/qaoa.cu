@@ -339,7 +339,8 @@ __global__ void __launch_bounds__(kQThreads)
 // amplitudes, and each layer computed its angles' sines again in FP64 by every
 // thread (65 us here, for 93 instances). Its float32 operations are kept, and so are their sums: a
 // thread's products of one group of 2^NB amplitudes add up in float32, everything
-// else in double. Rounds: bits 0..3, 4..7, 8..9, then 10..11 (the second pass).
+// else in double. Rounds of up to four bits: those below the tile width (10 where
+// none is given), then those from it on (the second pass).
 struct SmallLayout {
     uint32_t tl, cost, phase, mixer, emask, red, total;  // byte offsets behind psi
 };
@@ -419,7 +420,6 @@ __device__ __forceinline__ void small_rounds(float2 *tp, float2 *tl, uint32_t n,
         ph = nullptr;
     }
 }
-constexpr uint32_t kQSmallTile = 10;  // bits of the first pass
 
 __global__ void __launch_bounds__(kQThreads)
     k_qaoa_small(const QDesc *__restrict__ desc, const uint64_t *__restrict__ emasks, const double *__restrict__ gammas,
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(kQThreads)
         cost[x] = (uint8_t)cut_value(x, em, ne);
     }
     __syncthreads();
-    const uint32_t k = min(n, kQSmallTile);
+    const uint32_t k = min(n, D.k);  // bits of the first pass, as if in tiles of that width
     double none = 0.0;
     for (uint32_t l = 0; l < p; ++l) {
         const float4 m = mixer[l];
@@ -1101,14 +1101,14 @@ extern "C" int qf_qaoa_maxcut_batch(qf_ctx *ctx, const qf_qaoa_instance *inst, u
         return I.tile_qubits ? (int)I.tile_qubits : (opts && I.qubits <= 32 ? opts->tile_qubits[I.qubits] : 0);
     };
     auto batched = [&](const qf_qaoa_instance &I) { return I.qubits > (uint32_t)kQBTile && tile_req(I) == 0; };
-    auto rank = [&](const qf_qaoa_instance &I) { return batched(I) ? 0 : tile_req(I) ? 1 : 2; };
+    auto rank = [&](const qf_qaoa_instance &I) { return batched(I) ? 0 : I.qubits > (uint32_t)kQBTile ? 1 : 2; };
     std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) {
         const int ra = rank(inst[a]), rb = rank(inst[b]);
         if (ra != rb) return ra < rb;
         return inst[a].qubits > inst[b].qubits;
     });
     // rows [0, r_small): batched passes per qubit count (13..24 qubits); then
-    // one CTA per instance: rows of a given tile width, and from r_resident on
+    // one CTA per instance: rows of more than 12 qubits, and from r_resident on
     // those that stay in shared memory
     uint64_t amp_off = 0, cost_off = 0, ptab_off = 0, part_off = 0;
     uint32_t r_small = 0, r_resident = (uint32_t)n_inst, smem_resident = 0;
@@ -1125,14 +1125,15 @@ extern "C" int qf_qaoa_maxcut_batch(qf_ctx *ctx, const qf_qaoa_instance *inst, u
             ptab_off += 2ULL * p * (kQMaxEdges + 1);  // forward and reverse tables
             D.part = part_off;
             part_off += (uint64_t)(1 + 3 * p) << (D.n - kQBTile);
-        } else if (rank(I) == 2) {
-            r_resident = std::min(r_resident, (uint32_t)r);
-            smem_resident = std::max(smem_resident, small_layout(D.n, p, I.edge_count).total);
         } else {
-            const int kt = tile_req(I);
+            const int kt = tile_req(I) ? tile_req(I) : 10;
             D.k = (uint32_t)std::max(4, std::min(kQMaxTile, kt));
             if (D.n > D.k && D.n - D.k > D.k - 1) D.k = (D.n + 1) / 2 + 1;  // pass B needs n-k+1 <= k
             D.k = std::min<uint32_t>(D.k, (uint32_t)kQMaxTile);
+            if (rank(I) == 2) {
+                r_resident = std::min(r_resident, (uint32_t)r);
+                smem_resident = std::max(smem_resident, small_layout(D.n, p, I.edge_count).total);
+            }
         }
         D.e_begin = I.edge_begin;
         D.e_count = I.edge_count;
