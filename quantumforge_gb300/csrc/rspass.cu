@@ -107,9 +107,11 @@ __device__ __forceinline__ uint32_t layout_offset(uint32_t packed, int pos) { re
 // CZ: the pass has CZ gates. Their signs gather in a bit per amplitude and are
 // applied before the next op that mixes or moves amplitudes (20 qubits, 4 layers
 // with a CZ ring: 157 us of passes, now 127; passes without CZ ran 7 % slower with
-// the test for waiting signs, so they have a kernel without it).
+// the test for waiting signs, so they have a kernel without it). Three CTAs per
+// SM (80 registers): 22 qubits, 3 layers with a CNOT ring 459 us of passes with
+// two, 411 with three, 458 with four.
 template <int WB, bool CZ>
-__global__ void __launch_bounds__(32 << WB, (WB == 3 ? 2 : 1))
+__global__ void __launch_bounds__(32 << WB, (WB == 3 ? 3 : 1))
     k_rs_pass(float2 *__restrict__ amps, const RsPassArgs pa, const RsOp *__restrict__ g_ops,
               const double *__restrict__ g_mats) {
     constexpr int NT = 32 << WB;

@@ -5,11 +5,12 @@
 // GB300, 76 times below FP32), so a pass is priced by its FP64 instructions: two
 // per amplitude for a dense gate, none for CNOTs, CZs, X/Y/Z gates and SWAPs
 // (index and sign bookkeeping), four per thread for a phase on bits that a
-// thread's registers share. A 25-qubit depth-40 circuit takes 1805 of them per
-// amplitude and 107 ms, 97 % of the pipe's rate (the shared-memory interpreter:
-// 167 ms). complex64: instruction issue, 58 % of the slots, a third of them
-// arithmetic; a 21-qubit depth-40 circuit takes 0.82 ms (in-order register
-// interpreter: 1.43 ms).
+// thread's registers share. A 25-qubit depth-40 circuit takes 1715 of them per
+// amplitude and 104 ms, the pipe's rate (the shared-memory interpreter: 167 ms).
+// complex64: instruction issue, a fifth of it arithmetic, so a 21-qubit depth-40
+// circuit takes 0.54 ms (in-order register interpreter: 1.43 ms). Its kernel is
+// held to 64 registers, 32 warps per SM, although that spills 40 bytes: at 96
+// registers and 20 warps the circuit took 0.65 ms, at 80 and 24 0.58 ms.
 #pragma once
 
 #include <algorithm>
@@ -20,7 +21,7 @@ namespace qf {
 namespace vm {
 
 template <typename C, int R, bool DUAL>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, sizeof(C) == 8 && !DUAL ? 4 : 2)
     k_vm_pass(C *__restrict__ psi, C *__restrict__ lam, double *__restrict__ partials, uint32_t stride,
               const __grid_constant__ VmArgs a) {
     using T = typename Real<C>::T;
