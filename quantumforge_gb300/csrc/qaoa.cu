@@ -552,23 +552,61 @@ __device__ __forceinline__ void qb_load_cost(uint8_t *dst, const uint8_t *src, u
     for (uint32_t c = threadIdx.x; c < kQBT / 16; c += blockDim.x) qb_cp16(dst + 16 * c, src + (t << kQBTile) + 16 * c);
 }
 
-// C(x) for every amplitude of every instance of the class; per-layer phases
-// exp(-i gamma (W - 2c)) and mixer (cos beta, sin beta) as the per-instance
-// kernel computes them
+// C(x) for every amplitude of every instance of the class. Over a tile (its low 12
+// bits) the edges inside those bits count the same for every tile of the instance:
+// their bytes stay in the thread's registers over its CTA's run of tiles. An edge
+// from a low bit b to a high one adds x_b, or 1 - x_b where the high bit is set, one
+// between high bits a constant: per tile a constant c and D_b per low bit, found
+// by 13 threads. (56 us for 100 instances of 20 qubits, 156 with every edge
+// walked for every 16 amplitudes.)
 __global__ void __launch_bounds__(kQThreads)
     k_qaoa_costs(const QBArgs a, const QDesc *__restrict__ desc, const uint64_t *__restrict__ emasks, uint8_t *__restrict__ costs) {
-    __shared__ uint32_t em[kQMaxEdges];
-    const uint64_t items = (uint64_t)a.m * a.tiles;
-    for (uint64_t w = blockIdx.x; w < items; w += gridDim.x) {
-        const uint32_t ci = (uint32_t)(w >> (a.n - kQBTile));
-        const uint64_t t = (w & (a.tiles - 1));
-        const QDesc D = desc[a.r0 + ci];
+    __shared__ uint32_t low_e[kQMaxEdges], other_e[kQMaxEdges];
+    __shared__ uint32_t n_low, n_other;
+    __shared__ int lin[2][kQBTile + 1];  // D_b, then c
+    const uint64_t items = (uint64_t)a.m * a.tiles, w0 = blockIdx.x * a.chunk, w1 = min(items, w0 + a.chunk);
+    const uint32_t g = threadIdx.x;
+    uint32_t ci_now = ~0u, turn = 0;
+    uint4 low = make_uint4(0u, 0u, 0u, 0u);
+    uint64_t out = 0;
+    for (uint64_t w = w0; w < w1; ++w, turn ^= 1u) {
+        const uint32_t ci = (uint32_t)(w >> (a.n - kQBTile)), t = (uint32_t)(w & (a.tiles - 1));
+        if (ci != ci_now) {
+            const QDesc D = desc[a.r0 + ci];
+            __syncthreads();
+            if (g == 0) {
+                n_low = n_other = 0;
+                for (uint32_t e = 0; e < D.e_count; ++e) {
+                    const uint32_t m = (uint32_t)emasks[D.e_begin + e];
+                    if (m < kQBT) low_e[n_low++] = m;
+                    else other_e[n_other++] = m;
+                }
+            }
+            __syncthreads();
+            low = cut16(g << 4, low_e, n_low);
+            out = D.cost;
+            ci_now = ci;
+        }
+        if (g <= (uint32_t)kQBTile) {
+            int v = 0;
+            for (uint32_t e = 0; e < n_other; ++e) {
+                const uint32_t m = other_e[e], cut = __popc((m >> kQBTile) & t) & 1u;
+                if (g == (uint32_t)kQBTile) v += (int)cut;
+                else if ((m >> g) & 1u) v += cut ? -1 : 1;
+            }
+            lin[turn][g] = v;
+        }
         __syncthreads();
-        for (uint32_t e = threadIdx.x; e < D.e_count; e += blockDim.x) em[e] = (uint32_t)emasks[D.e_begin + e];
-        __syncthreads();
-        uint8_t *cost = costs + D.cost + (t << kQBTile);  // 16-byte aligned: batched rows come first, 2^n >= 2^13 each
-        for (uint32_t g = threadIdx.x; g < kQBT / 16; g += blockDim.x)
-            *reinterpret_cast<uint4 *>(cost + 16 * g) = cut16((uint32_t)(t << kQBTile) | (g << 4), em, D.e_count);
+        const int *D = lin[turn];
+        int h = D[kQBTile];
+#pragma unroll
+        for (uint32_t b = 4; b < (uint32_t)kQBTile; ++b) h += ((g >> (b - 4)) & 1u) ? D[b] : 0;
+        auto four = [&](int v) {
+            return (uint32_t)v | ((uint32_t)(v + D[0]) << 8) | ((uint32_t)(v + D[1]) << 16) | ((uint32_t)(v + D[0] + D[1]) << 24);
+        };
+        // 16-byte aligned: batched rows come first, 2^n >= 2^13 each
+        *reinterpret_cast<uint4 *>(costs + out + ((uint64_t)t << kQBTile) + 16 * g) =
+            make_uint4(low.x + four(h), low.y + four(h + D[2]), low.z + four(h + D[3]), low.w + four(h + D[2] + D[3]));
     }
 }
 
@@ -1233,7 +1271,7 @@ extern "C" int qf_qaoa_maxcut_batch(qf_ctx *ctx, const qf_qaoa_instance *inst, u
             const unsigned gfa = pass_grid(0, items, &cfa), gfb = pass_grid(rb, items, &cfb);
             const unsigned gra = pass_grid(4, items, &cra), grb = pass_grid(4 + rb, items, &crb);
             A.layer = 0;
-            A.chunk = 0;
+            A.chunk = cfa;
             k_qaoa_costs<<<gfa, kQThreads, 0, s>>>(A, d_desc, d_mask, d_costs);
             for (uint32_t l = 0; l < p; ++l) {
                 A.layer = l;

@@ -56,3 +56,27 @@ def test_graph_of_another_edge_count(backend):
         problems = [instance(rng, n, edges) for n in (14, 13, 12, 11, 10, 9)]
         got = QaoaBatch(problems, 2, backend=backend, use_graph=True).run(gam, bet)
         check(got, QaoaBatch(problems, 2, backend=backend, use_graph=False).run(gam, bet), problems)
+
+
+@pytest.mark.parametrize("n,count", [(13, 7), (14, 40), (16, 3)])
+@pytest.mark.parametrize("where", ["low", "high", "across", "any"])
+def test_cut_values_of_tiled_instances(backend, n, count, where):
+    """Edges inside a tile's low 12 bits, above them, between the two and mixed, more
+    runs of tiles than CTAs and fewer, against the oracle (tolerance as above)."""
+    rng = np.random.default_rng(n + count)
+    pairs = [(u, v) for u in range(n) for v in range(u)]
+    pairs = [(u, v) for u, v in pairs if where == "any" or where == ("low" if u < 12 else "high" if v >= 12 else "across")]
+    problems = []
+    for _ in range(count):
+        if pairs:
+            problems.append((n, [(*pairs[i], 1.0) for i in rng.permutation(len(pairs))[: int(rng.integers(1, 20))]]))
+    if not problems:
+        return
+    gam, bet = rng.uniform(0, np.pi, (len(problems), 1)), rng.uniform(-np.pi, np.pi, (len(problems), 1))
+    cost, grad = QaoaBatch(problems, 1, backend=backend).run(gam, bet)
+    for i in (0, len(problems) // 2, len(problems) - 1):
+        ed = problems[i][1]
+        e, g = O.adjoint_uncompute(W.qaoa_param_circuit(n, ed, 1), n, np.array([2 * gam[i, 0], 2 * bet[i, 0]]),
+                                   PauliSum.maxcut(ed).array())
+        tol = 16.0 * np.sqrt(2.0) * 2.0**-24 * (n + 1) * (len(ed) + 1)
+        assert abs(cost[i] - e) <= tol and np.abs(grad[i] - 2 * g).max() <= tol * (len(ed) + n + 1)
