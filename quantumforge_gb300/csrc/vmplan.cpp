@@ -1001,9 +1001,14 @@ struct Emitter {
         return QF_OK;
     }
     // One unitary part of a trajectory program: from layout `from` to exactly
-    // layout `to`, everything symbolic applied except the scalar (trajectories
-    // carry unnormalised states, and a global phase means nothing to them).
-    int segment(const PassSlots &slots, const Pass &p, const Layout &from, const Layout &to) {
+    // layout `to`, everything symbolic applied except the scalar: trajectories
+    // carry unnormalised states, and a global phase means nothing to them. Its
+    // magnitude tells how far the stored amplitudes have grown since their norm was
+    // last brought near one. A run with state-dependent steps does that itself
+    // (`measured`); otherwise it goes on to the next part, where emit_steps
+    // takes 2^-40 out once it is due. (1024 Hadamards between two measured runs
+    // would take the norm out of range.)
+    int segment(const PassSlots &slots, const Pass &p, const Layout &from, const Layout &to, bool measured) {
         pass = &p;
         ps = &slots;
         set_layout(from);
@@ -1019,7 +1024,9 @@ struct Emitter {
         if (!holds(to)) emit_remap(to);
         apply_terms(true);
         flush_phase_only();
+        const double grown = scale.abs();
         scale = Scalar();
+        if (!measured) scale *= grown;
         return QF_OK;
     }
     bool holds(const Layout &to) const {  // the amplitudes lie exactly as `to` has them
@@ -1169,7 +1176,7 @@ int vm_lower_trajectories(uint32_t n, const qf_op *ops, uint64_t n_ops, TrajProg
             for (int i = 0; i < slots.R; ++i) out.lreg[i] = slots.address_bit(at.rslot[i]);
         }
         r.rec_begin = (uint32_t)e.recs.size();
-        QF_TRY(e.segment(slots, p, at, to));
+        QF_TRY(e.segment(slots, p, at, to, r.n_sd > 0));
         r.n_recs = (uint32_t)e.recs.size() - r.rec_begin;
         at = to;
         uint8_t pos[64];

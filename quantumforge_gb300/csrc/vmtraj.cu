@@ -13,7 +13,8 @@
 //    index exchange. About 10 operations per amplitude and run, against 5.5 per
 //    channel when each channel reduces P(1) and the norm and rescales the state.
 //  * States stay unnormalised: a draw is compared as u N < p N, no division or
-//    square root of a norm; powers of two keep the range.
+//    square root of a norm; powers of two keep the range, taken out behind every run
+//    that finds the norm and, where none does, by the record streams.
 //  * One trajectory is simulated once: the one on which no event happens, but for
 //    the events that are certain. Every shot walks its own draws along that
 //    trajectory's thresholds and starts from the snapshot at the run of its first

@@ -50,3 +50,34 @@ def test_no_event_branch_without_weight(backend, n):
     for q in range(n):
         c.measure(q, 1 + q)
     check(c, n, shared_shots(n), 3 + n, backend)
+
+
+@pytest.mark.parametrize("n,shots", [(2, 60), (2, 5200), (4, 60), (4, 5200), (9, 60), (12, 60), (12, 400)])
+def test_depth_with_depolarizing_noise_alone(backend, n, shots):
+    """No channel depends on the state, so nothing but the gates' own factors tells how far
+    the stored amplitudes have grown: 1400 Hadamards."""
+    c = Circuit()
+    for _ in range(1400 // n):
+        for q in range(n):
+            c.push(Gate.H, q)
+            c.channel(q, NoiseChannel.Depolarizing(0.01))
+    for q in range(n):
+        c.push(Gate.Ry(0.5 + q), q)
+        c.measure(q, q)
+    check(c, n, shots, 1 + n, backend)
+
+
+@pytest.mark.parametrize("every", [1, 40, 300])
+def test_depth_with_a_damping_channel_now_and_then(backend, every):
+    """Runs that find the norm from the amplitudes between stretches that do not."""
+    n = 5
+    c = Circuit()
+    for i in range(1600):
+        q = i % n
+        c.push(Gate.H if i % 3 else Gate.Ry(0.1 * i), q)
+        c.channel(q, NoiseChannel.Depolarizing(0.005))
+        if i % every == every - 1:
+            c.channel(q, NoiseChannel.AmplitudeDamping(0.01))
+    for q in range(n):
+        c.measure(q, q)
+    check(c, n, shared_shots(n), 9, backend)
