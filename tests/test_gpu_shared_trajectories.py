@@ -6,6 +6,7 @@ import pytest
 
 import oracle as O
 from quantumforge_gb300 import Circuit, Gate, NoiseChannel
+from test_gpu_trajectories import noisy_circuit
 
 pytestmark = pytest.mark.gpu
 
@@ -81,3 +82,28 @@ def test_depth_with_a_damping_channel_now_and_then(backend, every):
     for q in range(n):
         c.measure(q, q)
     check(c, n, shared_shots(n), 9, backend)
+
+
+@pytest.mark.parametrize("strength", [0.01, 0.5])
+@pytest.mark.parametrize("n,layers,mid", [(2, 4, True), (3, 3, False), (5, 3, True), (6, 3, False), (7, 3, True), (8, 2, False),
+                                          (9, 2, True), (10, 2, False), (11, 2, True), (12, 2, False), (12, 2, True)])
+def test_shared_shots_match_literal_trajectories(backend, n, layers, mid, strength):
+    c = noisy_circuit(np.random.default_rng(7 * n + layers), n, layers, strength, mid)
+    check(c, n, shared_shots(n), 23 + n, backend)
+
+
+def test_more_runs_than_snapshots(backend):
+    """1100 runs (each iteration's CNOT acts on the qubit of the channel before it) of
+    64 KB each: shots start from every second run's amplitudes."""
+    n = 12
+    c = Circuit()
+    for i in range(1100):
+        q, before = 7 * i % n, 7 * (i - 1) % n
+        c.cnot(before, q)
+        c.push(Gate.Ry(0.3 + i), q)
+        c.channel(q, NoiseChannel.AmplitudeDamping(1e-3))
+        if i % 100 == 50:
+            c.measure(q, 20 + i // 100)
+    for q in range(n):
+        c.measure(q, q)
+    check(c, n, 400, 4, backend)
