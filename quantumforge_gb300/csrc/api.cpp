@@ -440,10 +440,12 @@ int normalize_state(qf_sv *sv) {
     return collapse(sv, 0, -1, norm);
 }
 
+// A Kraus operator.
 BGate mat1(uint32_t q, double m00, double m01, double m10, double m11) {
     BGate g;
     g.kind = BK_MAT1;
     g.q0 = q;
+    g.kraus = 1;
     g.m[0] = m00;
     g.m[2] = m01;
     g.m[4] = m10;

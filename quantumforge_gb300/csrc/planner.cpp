@@ -746,6 +746,7 @@ int plan_passes(uint32_t n, const std::vector<BGate> &gates, const PlanOpts &o, 
                     if (!varying || o.merge_any || matrix_is_diag(c) || matrix_is_cheap(c)) {
                         std::memcpy(taken[prev].g.m, c, sizeof c);
                         taken[prev].g.varying = varying;
+                        taken[prev].g.kraus |= it.g.kraus;
                         taken[prev].g.diag = matrix_is_diag(c);
                         taken[prev].g.op_index = -1;
                         return;

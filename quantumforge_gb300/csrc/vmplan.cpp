@@ -89,14 +89,17 @@ struct Sched {
 
 enum GClass : uint8_t { G_DENSE, G_DIAG, G_ANTI, G_CNOT, G_CZ, G_SWAP, G_OVZ, G_OVXY };
 
+// Up to the rounding of a product of gates. Kraus operators carry a flag: those of
+// a weak channel are as close to unitary as that.
 bool unit(cd f) { return std::abs(std::abs(f) - 1.0) < 1e-9; }
-bool anti_diagonal(const double m[8]) {  // a unitary one (not the jump operator of a damping channel)
-    return m[0] == 0 && m[1] == 0 && m[6] == 0 && m[7] == 0 && unit(cd(m[2], m[3])) && unit(cd(m[4], m[5]));
+bool anti_diagonal(const BGate &g) {  // a unitary one (not the jump operator of a damping channel)
+    const double *m = g.m;
+    return !g.kraus && m[0] == 0 && m[1] == 0 && m[6] == 0 && m[7] == 0 && unit(cd(m[2], m[3])) && unit(cd(m[4], m[5]));
 }
 
 GClass class_of(const BGate &g) {
     switch (g.kind) {
-    case BK_MAT1: return g.diag ? G_DIAG : anti_diagonal(g.m) ? G_ANTI : G_DENSE;
+    case BK_MAT1: return g.diag ? G_DIAG : anti_diagonal(g) ? G_ANTI : G_DENSE;
     case BK_CNOT: return G_CNOT;
     case BK_CZ: return G_CZ;
     case BK_SWAP: return G_SWAP;
@@ -704,7 +707,7 @@ struct Emitter {
         m[1] = -m[1];
         m[3] = -m[3];
     }
-    void emit_dense(uint32_t q, const double md[8]) {
+    void emit_dense(uint32_t q, const double md[8], bool kraus) {
         cd m[4] = {{md[0], md[1]}, {md[2], md[3]}, {md[4], md[5]}, {md[6], md[7]}};
         double mm[8];
         auto factor = [&] {
@@ -714,9 +717,9 @@ struct Emitter {
             }
             return factor_unitary_2x2(mm);
         };
-        Factored f = factor();
+        Factored f = kraus ? Factored() : factor();
         cd after(1.0, 0.0);
-        if (!f.ok) {
+        if (!f.ok && !kraus) {
             const double n0 = std::norm(m[0]) + std::norm(m[2]), n1 = std::norm(m[1]) + std::norm(m[3]);
             const cd dot = std::conj(m[0]) * m[1] + std::conj(m[2]) * m[3];
             const bool unitary = std::abs(n0 - 1.0) < 1e-9 && std::abs(n1 - 1.0) < 1e-9 && std::abs(dot) < 1e-9;
@@ -774,9 +777,9 @@ struct Emitter {
         zmask ^= adj[q];
         fn[ps->slot_of[q]].k ^= 1u;
     }
-    void emit_diag(uint32_t q, const double m[8]) {
+    void emit_diag(uint32_t q, const double m[8], bool kraus) {
         const cd a(m[0], m[1]), b(m[6], m[7]);
-        if (unit(a) && unit(b)) {
+        if (!kraus && unit(a) && unit(b)) {
             scale *= a;
             const cd f = b / a;
             if (f == cd(-1.0, 0.0)) zmask ^= 1ULL << q;
@@ -963,8 +966,8 @@ struct Emitter {
             const BGate &g = pass->gates[st.gate];
             const GClass c = class_of(g);
             switch (c) {
-            case G_DENSE: emit_dense(g.q0, g.m); --later[g.q0]; break;
-            case G_DIAG: emit_diag(g.q0, g.m); break;
+            case G_DENSE: emit_dense(g.q0, g.m, g.kraus); --later[g.q0]; break;
+            case G_DIAG: emit_diag(g.q0, g.m, g.kraus); break;
             case G_ANTI: emit_anti(g.q0, g.m); break;
             case G_CNOT: emit_cnot(g.q0, g.q1); break;
             case G_CZ: toggle(g.q0, g.q1); break;
