@@ -719,8 +719,8 @@ int plan_passes(uint32_t n, const std::vector<BGate> &gates, const PlanOpts &o, 
     // list's structure: a list of the same gate kinds, qubits, diagonal flags
     // and overlaps (new angles, shifted parameters, another optimiser step)
     // replays the recorded choices instead of searching again.
-    const std::string key = plan_key_of(n, k, low, o, items);
-    const PassChoices known = plan_cache_get(key);
+    const std::string key = o.recorded ? plan_key_of(n, k, low, o, items) : std::string();
+    const PassChoices known = o.recorded ? plan_cache_get(key) : nullptr;
     const bool hit = known != nullptr;
     std::vector<PassChoice> record;
     size_t pass_i = 0;
@@ -950,7 +950,7 @@ int plan_passes(uint32_t n, const std::vector<BGate> &gates, const PlanOpts &o, 
         p.a.n_slots = plan.n_slots - p.a.slot_base;
         plan.passes.push_back(std::move(p));
     }
-    if (!hit) plan_cache_put(key, std::move(record));
+    if (!hit && o.recorded) plan_cache_put(key, std::move(record));
     return QF_OK;
 }
 

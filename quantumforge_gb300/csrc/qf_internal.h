@@ -287,6 +287,7 @@ struct PlanOpts {
     bool backward = false;  // adjoint reverse sweep: inverse gates + overlaps
     int max_items = 768;    // bound on ops per pass (shared-memory budget)
     bool search = true;     // choose each pass's resident qubits by look-ahead
+    bool recorded = true;   // keep the choices for the next list of this structure (what a search costs)
     int block_qubits = 0;   // forward plans: fuse each pass's gates into dense blocks of up to this many
                             // qubits (2..5); every qubit a gate touches is then tile-resident
 };

@@ -1135,10 +1135,10 @@ int vm_lower_trajectories(uint32_t n, const qf_op *ops, uint64_t n_ops, TrajProg
         const std::vector<BGate> &gates = bound[pi];
         Pass p;
         p.resident = (1ULL << n) - 1;
-        if (!gates.empty()) {  // one-qubit runs merged
+        if (!gates.empty()) {  // one-qubit runs merged; hundreds of these plans would push the searched ones out
             PlanOpts po;
             po.tile_qubits = po.low_qubits = (int)n;
-            po.search = false;
+            po.search = po.recorded = false;
             po.vm = po.merge_any = true;
             po.max_items = 1 << 30;
             Plan merged;
