@@ -600,7 +600,7 @@ std::string plan_key_of(uint32_t n, int k, int low, const PlanOpts &o, const std
     put(n, 1);
     put((uint64_t)k, 1);
     put((uint64_t)low, 1);
-    put(o.merge_1q | (o.backward << 1) | (o.search << 2), 1);
+    put(o.merge_1q | (o.backward << 1) | (o.search << 2) | (o.merge_any << 3), 1);
     put((uint64_t)o.max_items, 4);
     put((uint64_t)o.block_qubits, 1);
     put(items.size(), 4);
