@@ -277,10 +277,7 @@ __device__ __forceinline__ bool decide_run(const TrajArgs &a, RunState &rs, cons
                 } else {
                     o = decide(s, draw(x), p1, norm, a.tie_eps, &bn, &ties);
                 }
-                if (bad_branch(bn, norm)) {
-                    rs.fault = 1;
-                    break;
-                }
+                if (bad_branch(bn, norm)) rs.fault = 1;
                 norm = bn;
                 const Outcome c = outcome_of(s, o);
                 const int e = rs.ex[j];
