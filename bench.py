@@ -809,7 +809,7 @@ def noise_shots(backend, cpu: bool, n: int = 12, shots: int = 100_000):
     t0 = time.perf_counter()
     got, width, ties = c.run_shots_packed(n, shots, seed, backend=backend, tie_eps=1e-12, noise=True)
     dt = time.perf_counter() - t0
-    out = {"qubits": n, "ops": len(c.operations), "shots": shots, "engine": "per-shot trajectories (k_trajectories)",
+    out = {"qubits": n, "ops": len(c.operations), "shots": shots, "engine": "per-shot trajectories (k_trajectory_runs)",
            "engine_call_s": dt, "engine_shots_per_s": shots / dt, "ties": int(ties),
            "distinct_outcomes": int(len(np.unique(got)))}
     t_shots = min(10_000, shots)
@@ -869,7 +869,7 @@ def qaoa_batch(backend, cpu: bool, count: int = 4096):
     peak, peak_kind = hbm_peak()
     out = {"instances": len(problems), "sizes": [12, 14, 16, 18, 20], "p": 4, "batch_s": dt,
            "instances_per_s": len(problems) / dt, "gradient_params_per_instance": 8, "tiles": tiles,
-           "tiles_meaning": "per qubit count: up to 12 the tile width of the one-CTA-per-instance kernel; above 12, "
+           "tiles_meaning": "per qubit count: up to 12 the bit at which the mixer's rounds are cut; above 12, "
                             "0 = batched tile passes, else one CTA per instance with that tile width",
            "autotune_s": t_tune, "dtype": "complex64", "host_copies_in_timing": True, "mean_cost": float(np.mean(cost)),
            "roofline": {"bound": "hbm", "algorithmic_gb": algo / 1e9, "achieved_gbs": algo / dt / 1e9, "peak": peak,

@@ -147,7 +147,10 @@ typedef struct qf_pauli_term {
 
 /* Amplitude storage type on the device. */
 enum qf_dtype {
-    QF_C64 = 0,   /* complex64: f32 re/im; gate arithmetic in f32, reductions in f64 */
+    QF_C64 = 0,   /* complex64: f32 re/im; gate arithmetic in f32, reductions in f64. The order of the f32
+                     operations depends on the engine that runs a list: qf_sv_apply_ops without parameters
+                     and inputs may take another one than the calls that return f64 results, and the two
+                     differ by f32 rounding */
     QF_C128 = 1   /* complex128: f64 re/im, the reference's precision */
 };
 
@@ -159,7 +162,7 @@ enum qf_exec_mode {
 };
 
 /* qf_exec_opts.flags */
-#define QF_EXEC_FLAG_SMEM_TILES 1  /* complex64: use the shared-memory tile kernel instead of register tiles */
+#define QF_EXEC_FLAG_SMEM_TILES 1  /* use the shared-memory tile kernel instead of register tiles (both dtypes) */
 #define QF_EXEC_FLAG_JIT 2         /* complex64: compile the plan's passes (NVRTC) even for small states */
 #define QF_EXEC_FLAG_NO_JIT 4      /* complex64: never compile passes; interpret them */
 #define QF_EXEC_FLAG_SHOTS_TREE 8  /* shots: always walk the branch tree of device states */
@@ -234,6 +237,9 @@ int qf_ctx_create(int device, qf_ctx **out);
 int qf_ctx_destroy(qf_ctx *ctx);
 /* CudaDeviceStateBatch::synchronize (src/cuda.rs:1792). */
 int qf_ctx_synchronize(qf_ctx *ctx);
+/* A context keeps up to 256 MB of the memory of destroyed states for new ones of
+ * the same size (states whose address was given out excepted); it goes back to
+ * the device when any context's allocation fails, and with the context. */
 /* Raw stream handle (a cudaStream_t) of the context, for callers that order
  * their own work after the engine's. */
 int qf_ctx_stream(qf_ctx *ctx, void **stream_out);

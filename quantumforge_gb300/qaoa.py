@@ -5,10 +5,10 @@ expected cut of the QAOA state
 (``maxcut_qaoa_expectation``, src/qaoa_transfer.rs:221-236, on the circuit of
 ``algorithms::qaoa_maxcut``, src/algorithms.rs:110-137, unit weights) and its
 exact gradient with respect to every gamma_l and beta_l: instances of up to 12
-qubits one CTA each, larger ones (up to 24) as tile passes batched over all
-instances of a qubit count, or one CTA each when asked. ``autotune_tiles``
-picks, per qubit count, the shared-memory tile width of the small instances
-and, above 12 qubits, batched passes or one CTA per instance, by timing
+qubits one CTA each, wholly in shared memory, larger ones (up to 24) as tile
+passes batched over all instances of a qubit count, or one CTA each when asked.
+``autotune_tiles`` picks, per qubit count, where the mixer of the small instances
+is cut and, above 12 qubits, batched passes or one CTA per instance, by timing
 sub-batches; ``save_tiles`` / ``load_tiles`` persist the table.
 """
 from __future__ import annotations
@@ -85,10 +85,12 @@ class QaoaBatch:
 def autotune_tiles(problems, p: int, candidates=(8, 9, 10, 11, 12), reps: int = 2, backend=None,
                    large_candidates=(0, 12, 11), max_large: int = 24) -> dict:
     """Best execution per qubit count, timed on the sub-batch of that count
-    (at most 256 instances). Up to 12 qubits: the tile width of the
-    one-CTA-per-instance kernel, from `candidates`. Above 12 (up to
-    `max_large`): 0 = batched tile passes over every instance of the count, or
-    one CTA per instance with tiles of a width in `large_candidates`."""
+    (at most 256 instances). Up to 12 qubits an instance stays in shared memory at
+    any width: the one taken from `candidates` only says which bit the mixer's
+    rounds of up to four bits are cut at, and moves time and results by little.
+    Above 12 (up to `max_large`): 0 = batched tile passes over every instance of
+    the count, or one CTA per instance with tiles of a width in
+    `large_candidates`."""
     rng = np.random.default_rng(0)
     best = {}
     by_n: dict[int, list] = {}
